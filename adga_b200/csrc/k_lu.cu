@@ -3,9 +3,9 @@
 //
 // Per step J (panel width NB):
 //   k_panel      one CTA per matrix factors rows J..N of the NB panel columns
-//                in 8-column sub-panels held in registers (pivot search,
+//                in 2- to 16-column sub-panels held in registers (pivot search,
 //                row swap and rank-1 updates never leave the SM), with
-//                right-looking rank-8 updates of the rest of the panel;
+//                right-looking updates of the rest of the panel;
 //   k_triinv     inverts the unit-lower and upper NB x NB diagonal blocks;
 //   k_swap_trsm  applies the panel's row interchanges to the other columns
 //                and forms U12 = L11^-1 A12 as a small GEMM;
@@ -13,323 +13,447 @@
 //                BF16x3 kernel of the mixed path).
 // Pivot choice follows izamax: the largest |re|+|im|, the lowest row on ties.
 #include "lu.cuh"
+#include <algorithm>
 #include <climits>
 
-#define SWD 8          // sub-panel width
-#define MAXNB 128      // largest outer panel width
 
 // ---------------------------------------------------------------------------
-template <int RPT> struct PanelThreads { static constexpr int v = RPT == 1 ? 1024 : RPT == 2 ? 640 : 512; };
-
-template <typename T> struct PanelShared {
-  typename cx<T>::real red_v[32];
-  int red_i[32];
-  int s_p;
-  int s_info;
-  int s_piv[SWD];
-  int mdst[2 * SWD], msrc[2 * SWD];
-  int mcnt;
-  T bufP[SWD], bufC[SWD];
-  T Lss[SWD * SWD];
-  T Us[SWD * MAXNB];
+// Panel factorisation, one CTA per matrix: SW-column sub-panels live in
+// registers (thread t owns rows J + t + q nt), and the rest of the panel takes
+// their interchanges, triangular solve and rank-SW update from global memory.
+//
+// Bound by the serial chain of a column: the pivot search is three integer
+// warp reductions over the bit pattern of |re|+|im| (high word, low word, then
+// the lowest row), every warp's candidate row is put in shared memory beside
+// its key before the one barrier of the column, and after it every warp
+// reduces the candidates itself, so that neither a second reduction stage nor
+// a row broadcast needs another barrier.  The buffers alternate with the
+// column's parity.  Sub-panels of 16 columns where one row per thread fits
+// (rows <= 512: half the passes over the rest of the panel), else of 8 and less.
+// With double-precision shuffles, three barriers a column and a serially
+// composed interchange map: 137 us for a 40 x 40 panel, 417 us for 1016 x 64,
+// 1799 us for 500 of them; this form: 66 us, 250 us and 1182 us.
+// ---------------------------------------------------------------------------
+template <typename T, int SW> struct PanelShared {
+  unsigned long long key[2][32];
+  int row[2][32];
+  T cand[2][32][SW];           // each warp's candidate row
+  T crow[2][SW];               // the row at the diagonal
+  T Lss[SW * SW];
+  int piv[SW], dst[2 * SW], src[2 * SW], cnt;
 };
 
-// One column CC of the register-resident sub-panel: pivot search, row swap,
-// scaling and rank-1 update.  CC is a compile-time constant so that every
-// index into the register array a[][] is static.
-template <typename T, int RPT, int CC>
-__device__ __forceinline__ void panel_column(T (&a)[RPT][SWD], PanelShared<T> &S, int J, int N,
-                                             int c0, int sw, int t, int nt) {
-  typedef typename cx<T>::real R;
-  if (CC >= sw) return;
-  const int lane = t & 31, warp = t >> 5, nw = nt >> 5;
-  const int col = c0 + CC;
-  R best = R(-1);
-  int bidx = INT_MAX;
-#pragma unroll
-  for (int q = 0; q < RPT; ++q) {
-    const int r = J + t + q * nt;
-    if (r >= col && r < N) {
-      R v = cabs1(a[q][CC]);
-      if (v > best) { best = v; bidx = r; }
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    R ov = __shfl_xor_sync(0xffffffffu, best, o);
-    int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
-    if (ov > best || (ov == best && oi < bidx)) { best = ov; bidx = oi; }
-  }
-  if (lane == 0) { S.red_v[warp] = best; S.red_i[warp] = bidx; }
-  __syncthreads();
-  if (warp == 0) {
-    best = lane < nw ? S.red_v[lane] : R(-1);
-    bidx = lane < nw ? S.red_i[lane] : INT_MAX;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      R ov = __shfl_xor_sync(0xffffffffu, best, o);
-      int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
-      if (ov > best || (ov == best && oi < bidx)) { best = ov; bidx = oi; }
-    }
-    if (lane == 0) S.s_p = (bidx == INT_MAX || bidx < col || bidx >= N) ? col : bidx;
-  }
-  __syncthreads();
-  const int p = S.s_p;
-  const int oc = col - J, op = p - J;
-  const bool own_c = (oc % nt) == t, own_p = (op % nt) == t;
-  const int qc = oc / nt, qp = op / nt;
-#pragma unroll
-  for (int q = 0; q < RPT; ++q) {
-    if (own_p && q == qp)
-#pragma unroll
-      for (int c2 = 0; c2 < SWD; ++c2) S.bufP[c2] = a[q][c2];
-    if (own_c && q == qc)
-#pragma unroll
-      for (int c2 = 0; c2 < SWD; ++c2) S.bufC[c2] = a[q][c2];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < RPT; ++q) {
-    if (own_c && q == qc)
-#pragma unroll
-      for (int c2 = 0; c2 < SWD; ++c2) a[q][c2] = S.bufP[c2];
-    if (own_p && p != col && q == qp)
-#pragma unroll
-      for (int c2 = 0; c2 < SWD; ++c2) a[q][c2] = S.bufC[c2];
-  }
-  const T piv = S.bufP[CC];
-  const bool zero = (piv.x == R(0) && piv.y == R(0));
-  if (zero && t == 0 && S.s_info == 0) S.s_info = col + 1;
-  const T rcp = zero ? czero<T>() : crcp(piv);
-  T prow[SWD];
-#pragma unroll
-  for (int c2 = CC + 1; c2 < SWD; ++c2) prow[c2] = S.bufP[c2];
-#pragma unroll
-  for (int q = 0; q < RPT; ++q) {
-    const int r = J + t + q * nt;
-    if (r > col && r < N) {
-      const T l = zero ? a[q][CC] : cmul(a[q][CC], rcp);
-      a[q][CC] = l;
-#pragma unroll
-      for (int c2 = CC + 1; c2 < SWD; ++c2)
-        if (c2 < sw) cfms(a[q][c2], l, prow[c2]);
-    }
-  }
-  if (t == 0) S.s_piv[CC] = p;
+// the largest key of the warp and the lowest row that holds it (keys 0: none)
+__device__ __forceinline__ void warp_argmax(unsigned long long &key, int &row) {
+  const unsigned hi = (unsigned)(key >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = hi == mh ? (unsigned)key : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
+  const unsigned long long m = ((unsigned long long)mh << 32) | ml;
+  row = (int)__reduce_min_sync(0xffffffffu, (key == m && m) ? (unsigned)row : (unsigned)INT_MAX);
+  key = m;
 }
 
-template <typename T, int RPT>
-__global__ void __launch_bounds__(PanelThreads<RPT>::v, 1)
+// 1 / z with one division: z scaled by a power of two so that |z|^2 lies in [1, 32) (or below,
+// for subnormal z), exact up to the rounding of |z|^2, of the division and of the products
+__device__ __forceinline__ z64 crcp_scaled(z64 z) {
+  const int e = max(__double2hiint(z.x) & 0x7ff00000, __double2hiint(z.y) & 0x7ff00000);
+  const double s = __hiloint2double(max(0x7fe00000 - e, 0x00100000), 0);
+  const double a = z.x * s, b = z.y * s;
+  const double f = __drcp_rn(fma(a, a, b * b));
+  return make_double2(a * f * s, -b * f * s);
+}
+__device__ __forceinline__ z32 crcp_scaled(z32 z) { return crcp(z); }
+
+// One column CC of the register-resident sub-panel.  CC is a compile-time
+// constant so that every index into the register array is static.
+template <typename T, int RPT, int SW, int CC>
+__device__ __forceinline__ void panel_column(T (&a)[RPT][SW], PanelShared<T, SW> &S, int J, int N, int c0, int sw,
+                                             int t, int nt, int *ipiv, int &info) {
+  if (CC >= sw) return;
+  const int lane = t & 31, warp = t >> 5, nw = nt >> 5, par = CC & 1;
+  const int col = c0 + CC;
+  unsigned long long key = 0;
+  int row = INT_MAX;
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int r = J + t + q * nt;
+    const double v = (double)cabs1(a[q][CC]);
+    // 1 + the bits of a non-negative number order like the number; NaN is never a pivot
+    const unsigned long long k = (r >= col && r < N && v == v) ? (unsigned long long)__double_as_longlong(v) + 1 : 0;
+    if (k > key) { key = k; row = r; }
+  }
+  const int mine = row;
+  warp_argmax(key, row);
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int r = J + t + q * nt;
+    if (key && r == row && mine == row)
+#pragma unroll
+      for (int c2 = 0; c2 < SW; ++c2) S.cand[par][warp][c2] = a[q][c2];
+    if (r == col)
+#pragma unroll
+      for (int c2 = 0; c2 < SW; ++c2) S.crow[par][c2] = a[q][c2];
+  }
+  if (lane == 0) { S.key[par][warp] = key; S.row[par][warp] = row; }
+  __syncthreads();
+  unsigned long long k2 = lane < nw ? S.key[par][lane] : 0;
+  int p = lane < nw ? S.row[par][lane] : INT_MAX;
+  const int rl = p;
+  warp_argmax(k2, p);
+  const unsigned who = __ballot_sync(0xffffffffu, k2 && rl == p && lane < nw);
+  const T *prow = who ? S.cand[par][__ffs(who) - 1] : S.crow[par];
+  if (!who) p = col;                       // no eligible row (all NaN)
+  const T piv = prow[CC];
+  const bool zero = piv.x == 0 && piv.y == 0;
+  if (zero && info == 0) info = col + 1;
+  const T rcp = zero ? czero<T>() : crcp_scaled(piv);
+  if (p != col) {
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      const int r = J + t + q * nt;
+      if (r == col)
+#pragma unroll
+        for (int c2 = 0; c2 < SW; ++c2) a[q][c2] = prow[c2];
+      else if (r == p)
+#pragma unroll
+        for (int c2 = 0; c2 < SW; ++c2) a[q][c2] = S.crow[par][c2];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    if (J + t + q * nt > col) {            // rows past N hold zeros
+      if (!zero) a[q][CC] = cmul(a[q][CC], rcp);
+#pragma unroll
+      for (int c2 = CC + 1; c2 < SW; ++c2) cfms(a[q][c2], a[q][CC], prow[c2]);
+    }
+  }
+  if (t == 0) { S.piv[CC] = p; ipiv[col] = p; }
+}
+
+template <typename T, int RPT, int SW, int CC>
+__device__ __forceinline__ void panel_columns(T (&a)[RPT][SW], PanelShared<T, SW> &S, int J, int N, int c0, int sw,
+                                              int t, int nt, int *ipiv, int &info) {
+  if constexpr (CC < SW) {
+    panel_column<T, RPT, SW, CC>(a, S, J, N, c0, sw, t, nt, ipiv, info);
+    panel_columns<T, RPT, SW, CC + 1>(a, S, J, N, c0, sw, t, nt, ipiv, info);
+  }
+}
+
+template <typename T, int RPT, int SW, int NTMAX>
+__global__ void __launch_bounds__(NTMAX, 1)
 k_panel(T *M, size_t strideM, int N, int J, int jb, int *ipiv_all, int *info_all) {
   const int b = blockIdx.x;
   T *A = M + (size_t)b * strideM;
   int *ipiv = ipiv_all + (size_t)b * N;
   const int nt = blockDim.x, t = threadIdx.x;
-  __shared__ PanelShared<T> S;
+  __shared__ PanelShared<T, SW> S;
   extern __shared__ __align__(16) unsigned char panel_dyn[];
-  T *Gs = reinterpret_cast<T *>(panel_dyn);        // [MAXNB][2*SWD] interchange buffer
-  if (t == 0) S.s_info = info_all[b];
-  T a[RPT][SWD];
+  T *Gs = reinterpret_cast<T *>(panel_dyn);        // [jb - sw columns][2 SW]: moved rows, then U in the first SW
+  int info = info_all[b];
+  T a[RPT][SW];
 
-  for (int s = 0; s < jb; s += SWD) {
-    const int sw = min(SWD, jb - s), c0 = J + s;
+#pragma unroll 1
+  for (int s = 0; s < jb; s += SW) {
+    const int sw = min(SW, jb - s), c0 = J + s;
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
       const int r = J + t + q * nt;
 #pragma unroll
-      for (int cc = 0; cc < SWD; ++cc)
+      for (int cc = 0; cc < SW; ++cc)
         a[q][cc] = (r >= c0 && r < N && cc < sw) ? A[r + (size_t)(c0 + cc) * N] : czero<T>();
     }
-    panel_column<T, RPT, 0>(a, S, J, N, c0, sw, t, nt);
-    panel_column<T, RPT, 1>(a, S, J, N, c0, sw, t, nt);
-    panel_column<T, RPT, 2>(a, S, J, N, c0, sw, t, nt);
-    panel_column<T, RPT, 3>(a, S, J, N, c0, sw, t, nt);
-    panel_column<T, RPT, 4>(a, S, J, N, c0, sw, t, nt);
-    panel_column<T, RPT, 5>(a, S, J, N, c0, sw, t, nt);
-    panel_column<T, RPT, 6>(a, S, J, N, c0, sw, t, nt);
-    panel_column<T, RPT, 7>(a, S, J, N, c0, sw, t, nt);
-    // ---- write the sub-panel back; keep its L block for the TRSM below
+    panel_columns<T, RPT, SW, 0>(a, S, J, N, c0, sw, t, nt, ipiv, info);
+    // the sub-panel back to the matrix; its L block for the solve below
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
       const int r = J + t + q * nt;
       if (r >= c0 && r < N) {
 #pragma unroll
-        for (int cc = 0; cc < SWD; ++cc)
+        for (int cc = 0; cc < SW; ++cc)
           if (cc < sw) A[r + (size_t)(c0 + cc) * N] = a[q][cc];
         const int i = r - c0;
-        if (i < sw)
+        if (i < SW)
 #pragma unroll
-          for (int cc = 0; cc < SWD; ++cc) S.Lss[i + cc * SWD] = a[q][cc];
+          for (int cc = 0; cc < SW; ++cc) S.Lss[i + cc * SW] = a[q][cc];
       }
     }
-    if (t == 0) {
-      // compose the sub-panel's interchanges into a (dst <- src) row map
-      int keys[2 * SWD], cont[2 * SWD], nk = sw;
-      for (int i = 0; i < sw; ++i) { keys[i] = c0 + i; cont[i] = c0 + i; }
-      for (int i = 0; i < sw; ++i) {
-        const int p = S.s_piv[i];
-        if (p == c0 + i) continue;
-        int k = -1;
-        if (p < c0 + sw) k = p - c0;
-        else {
-          for (int q = sw; q < nk; ++q)
-            if (keys[q] == p) { k = q; break; }
-          if (k < 0) { k = nk++; keys[k] = p; cont[k] = p; }
-        }
-        const int x = cont[i]; cont[i] = cont[k]; cont[k] = x;
+    if (jb == sw) break;                           // the panel is this sub-panel
+    __syncthreads();                               // S.piv complete
+    if (t < 32) {
+      // the interchanges as (dst <- src): the sub-panel's positions, then the other touched rows
+      const int me = t % SW;
+      const bool top = t < SW;
+      const int pos = top ? c0 + me : S.piv[me];
+      bool use = t < 2 * SW && me < sw && (top || pos >= c0 + sw);
+      int x = pos;
+#pragma unroll
+      for (int i = SW - 1; i >= 0; --i) {
+        if (i >= sw) continue;
+        const int p = S.piv[i];
+        if (x == c0 + i) x = p;
+        else if (x == p) x = c0 + i;
+        if (!top && i < me && p == pos) use = false;       // listed already
       }
-      int cnt = 0;
-      for (int k = 0; k < nk; ++k)
-        if (cont[k] != keys[k]) { S.mdst[cnt] = keys[k]; S.msrc[cnt] = cont[k]; ++cnt; }
-      S.mcnt = cnt;
+      const unsigned m = __ballot_sync(0xffffffffu, use);
+      if (use) {
+        const int k = __popc(m & ((1u << t) - 1));
+        S.dst[k] = pos;
+        S.src[k] = x;
+      }
+      if (t == 0) S.cnt = __popc(m);
     }
     __syncthreads();
-    if (t < sw) ipiv[c0 + t] = S.s_piv[t];
-    // ---- apply the sub-panel's interchanges to the other panel columns:
-    //      every (row, column) load into shared memory, a barrier, every store
-    const int nother = jb - sw, mc = S.mcnt;
+    // the touched rows of the other panel columns, and the rows of U to solve: every load before a
+    // barrier, every store after it
+    const int nother = jb - sw, mc = S.cnt;
+#pragma unroll 2
     for (int e = t; e < nother * mc; e += nt) {
-      const int u = e / mc, k = e % mc;
-      const int col = (u < s) ? J + u : c0 + sw + (u - s);
-      Gs[u * 2 * SWD + k] = A[(size_t)S.msrc[k] + (size_t)col * N];
+      const int u = e / mc, k = e - u * mc;
+      const int col = u < s ? J + u : c0 + sw + (u - s);
+      Gs[u * 2 * SW + k] = A[(size_t)S.src[k] + (size_t)col * N];
     }
     __syncthreads();
-    for (int e = t; e < nother * mc; e += nt) {
-      const int u = e / mc, k = e % mc;
-      const int col = (u < s) ? J + u : c0 + sw + (u - s);
-      A[(size_t)S.mdst[k] + (size_t)col * N] = Gs[u * 2 * SWD + k];
-    }
-    __syncthreads();
-    // ---- U rows of the right panel columns: unit-lower solve with Lss
     const int nright = jb - s - sw;
-    for (int u = t; u < nright; u += nt) {
-      const int col = c0 + sw + u;
-      T *Ac = A + (size_t)col * N;
-      T x[SWD];
+#pragma unroll 2
+    for (int e = t; e < nother * mc; e += nt) {
+      const int u = e / mc, k = e - u * mc;
+      const int col = u < s ? J + u : c0 + sw + (u - s);
+      if (u < s ? S.src[k] != S.dst[k] : k >= sw) A[(size_t)S.dst[k] + (size_t)col * N] = Gs[u * 2 * SW + k];
+    }
+    // U rows of the right panel columns: unit-lower solve with Lss, one thread a column
+    for (int u = nt - 1 - t; u < nright; u += nt) {
+      T *g = Gs + (s + u) * 2 * SW, *Ac = A + c0 + (size_t)(c0 + sw + u) * N;
+      // columns are left, so sw == SW; in blocks of at most 8 rows (registers)
+      constexpr int HB = SW < 8 ? SW : 8;
+#pragma unroll 1
+      for (int h = 0; h < SW; h += HB) {
+        T x[HB];
 #pragma unroll
-      for (int i = 0; i < SWD; ++i) x[i] = (i < sw) ? Ac[c0 + i] : czero<T>();
+        for (int i = 0; i < HB; ++i) x[i] = g[h + i];
+#pragma unroll 1
+        for (int k = 0; k < h; ++k) {
+          const T y = g[k];
 #pragma unroll
-      for (int i = 1; i < SWD; ++i)
+          for (int i = 0; i < HB; ++i) cfms(x[i], S.Lss[h + i + k * SW], y);
+        }
 #pragma unroll
-        for (int k = 0; k < i; ++k) cfms(x[i], S.Lss[i + k * SWD], x[k]);
+        for (int k = 0; k < HB - 1; ++k)
 #pragma unroll
-      for (int i = 0; i < SWD; ++i)
-        if (i < sw) { Ac[c0 + i] = x[i]; S.Us[i * MAXNB + u] = x[i]; }
+          for (int i = k + 1; i < HB; ++i) cfms(x[i], S.Lss[h + i + (h + k) * SW], x[k]);
+#pragma unroll
+        for (int i = 0; i < HB; ++i) { Ac[h + i] = x[i]; g[h + i] = x[i]; }
+      }
     }
     __syncthreads();
-    // ---- rank-sw update of the rows below, right panel columns, in chunks of
-    //      CW columns whose loads are all issued before their stores (CW
-    //      keeps the chunk beside a[][] inside the register budget)
+    // rank-SW update of the rows below, right panel columns, in chunks of CW columns whose loads are
+    // all issued before their stores (a full sub-panel: sw == SW whenever columns are left)
     if (nright > 0) {
+      constexpr int CW = sizeof(T) == 8 ? 4 : (RPT == 1 ? 4 : 2);
+      const T *U = Gs + s * 2 * SW;
+      T *arow = A + J + t + (size_t)(c0 + sw) * N;
+#pragma unroll 1
+      for (int u0 = 0; u0 < nright; u0 += CW) {
+        T v[RPT][CW];
 #pragma unroll
-      for (int q = 0; q < RPT; ++q) {
-        const int r = J + t + q * nt;
-        if (r >= c0 + sw && r < N) {
-          T *arow = A + r + (size_t)(c0 + sw) * N;
-          constexpr int CW = sizeof(T) == 8 ? 4 : 2;
-          for (int u0 = 0; u0 < nright; u0 += CW) {
-            T v[CW];
-#pragma unroll
-            for (int j = 0; j < CW; ++j)
-              if (u0 + j < nright) v[j] = arow[(size_t)(u0 + j) * N];
-#pragma unroll
-            for (int j = 0; j < CW; ++j)
-#pragma unroll
-              for (int i = 0; i < SWD; ++i)
-                if (i < sw) cfms(v[j], a[q][i], S.Us[i * MAXNB + u0 + j]);
+        for (int q = 0; q < RPT; ++q) {
+          const int r = J + t + q * nt;
+          if (r >= c0 + sw && r < N)
 #pragma unroll
             for (int j = 0; j < CW; ++j)
-              if (u0 + j < nright) arow[(size_t)(u0 + j) * N] = v[j];
+              if (u0 + j < nright) v[q][j] = arow[q * nt + (size_t)(u0 + j) * N];
+        }
+#pragma unroll
+        for (int j = 0; j < CW; ++j)
+#pragma unroll
+          for (int i = 0; i < SW; ++i) {
+            const T y = U[(u0 + j) * 2 * SW + i];
+#pragma unroll
+            for (int q = 0; q < RPT; ++q) cfms(v[q][j], a[q][i], y);
           }
+#pragma unroll
+        for (int q = 0; q < RPT; ++q) {
+          const int r = J + t + q * nt;
+          if (r >= c0 + sw && r < N)
+#pragma unroll
+            for (int j = 0; j < CW; ++j)
+              if (u0 + j < nright) arow[q * nt + (size_t)(u0 + j) * N] = v[q][j];
         }
       }
     }
     __syncthreads();
   }
-  if (t == 0) info_all[b] = S.s_info;
+  if (t == 0) info_all[b] = info;
 }
 
 // ---------------------------------------------------------------------------
-// Inverses of the diagonal block: strictly-lower part -> unit-lower inverse
-// (columns right to left), upper part -> upper inverse (columns left to right),
-// both in place in shared memory as LAPACK's xTRTI2 does.
+// Inverses of the step's diagonal block, unit-lower L11^-1 and upper U11^-1,
+// and the step's interchanges as one row map.
+//
+// One CTA per matrix, bound by latency (a 64 x 64 block is 175k complex FMAs).
+// Both inverses live in the factored block's own array: strictly lower part
+// L^-1, upper part U^-1.  Eight warps invert the 16 x 16 diagonal blocks of
+// the two triangles (lane = column, right-looking so that the updates of a
+// column step are independent), then two levels of recursive doubling join
+// them, X10 = -X11 (L10 X00) and Y01 = -Y00 (U01 Y11), the inner product
+// taking the place of L10 / U01.  Blocks wholly outside jb are skipped.  66 KB
+// of shared memory in FP64: three CTAs per SM.
+// The row map: the content of position x after the interchanges (J+i <-> p_i,
+// in order) came from the position reached by undoing them from the last to
+// the first, one thread per touched position.
+// Column by column through shared memory (xTRTI2's order) with the map
+// composed by one thread: 187 us on a single 64 x 64 block, 391 us per step of
+// 500 blocks; this form: 30 us and 74 us.
 // ---------------------------------------------------------------------------
+constexpr int TI_LD = 65;
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 3)
 k_triinv(const T *M, size_t strideM, int N, int J, int jb, int NB, int nsteps, T *Linv, T *Uinv,
          const int *ipiv_all, int *rmap_all) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  T *D = reinterpret_cast<T *>(smraw);
-  T *tmp = D + NB * NB;
-  __shared__ T s_d;
-  __shared__ int keys[2 * MAXNB], content[2 * MAXNB];
-  const int b = blockIdx.x, t = threadIdx.x, nt = blockDim.x;
+  T *D = reinterpret_cast<T *>(smraw);          // [64][TI_LD], column-major
+  __shared__ T rcps[64];
+  __shared__ int piv[64], s_cnt;
+  const int b = blockIdx.x, t = threadIdx.x, w = t >> 5, lane = t & 31;
   const T *A = M + (size_t)b * strideM;
-  const int n = jb;
-  if (t == 0) {
-    // compose the step's interchanges (row J+i <-> ipiv[J+i], in order) into
-    // one map over the rows they touch
-    const int *ip = ipiv_all + (size_t)b * N + J;
-    int nk = jb;
-    for (int i = 0; i < jb; ++i) { keys[i] = J + i; content[i] = J + i; }
-    for (int i = 0; i < jb; ++i) {
-      const int p = ip[i];
-      if (p == J + i) continue;
-      int k;
-      if (p < J + jb) {
-        k = p - J;
-      } else {
-        k = -1;
-        for (int q = jb; q < nk; ++q)
-          if (keys[q] == p) { k = q; break; }
-        if (k < 0) { k = nk++; keys[k] = p; content[k] = p; }
-      }
-      const int x = content[i]; content[i] = content[k]; content[k] = x;
-    }
-    int *rm = rmap_all + (size_t)b * RMAP_STRIDE;
-    int cnt = 0;
-    for (int k = 0; k < nk; ++k)
-      if (content[k] != keys[k]) { rm[1 + 2 * cnt] = keys[k]; rm[2 + 2 * cnt] = content[k]; ++cnt; }
-    rm[0] = cnt;
+  const T one = cx<T>::make(1, 0), zero = czero<T>();
+#pragma unroll 4
+  for (int e = t; e < 64 * 64; e += 256) {
+    const int i = e & 63, j = e >> 6;           // identity outside the jb x jb block
+    D[i + j * TI_LD] = (i < jb && j < jb) ? A[(size_t)(J + i) + (size_t)(J + j) * N] : (i == j ? one : zero);
   }
-  for (int e = t; e < n * n; e += nt) {
-    int i = e % n, j = e / n;
-    D[i + j * NB] = A[(size_t)(J + i) + (size_t)(J + j) * N];
+  if (t < jb) piv[t] = ipiv_all[(size_t)b * N + J + t];
+  if (t == 0) s_cnt = 0;
+  __syncthreads();
+  if (t < 64) rcps[t] = crcp(D[t + t * TI_LD]);
+  if (t >= 128 && (t & 63) < jb) {
+    // warps 4..7: positions J + i (t < 192) and the pivots' own rows below the block
+    const int me = t & 63, pos = t < 192 ? J + me : piv[me];
+    bool use = t < 192 || pos >= J + jb;
+    int x = pos;
+    for (int i = jb - 1; i >= 0; --i) {
+      const int p = piv[i];
+      if (x == J + i) x = p;
+      else if (x == p) x = J + i;
+      if (t >= 192 && i < me && p == pos) use = false;     // listed by an earlier interchange
+    }
+    if (use && x != pos) {
+      const int k = atomicAdd(&s_cnt, 1);
+      int *rm = rmap_all + (size_t)b * RMAP_STRIDE;
+      rm[1 + 2 * k] = pos;
+      rm[2 + 2 * k] = x;
+    }
   }
   __syncthreads();
-  for (int j = n - 2; j >= 0; --j) {
-    for (int i = j + 1 + t; i < n; i += nt) tmp[i] = D[i + j * NB];
+  if (t == 0) rmap_all[(size_t)b * RMAP_STRIDE] = s_cnt;
+  const int o16 = 16 * (w & 3);
+  if (o16 < jb && lane < 16) {
+    const int l = lane;
+    T x[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) x[r] = r == l ? one : zero;
+    const T *B = D + o16 + o16 * TI_LD;
+    if (w < 4) {
+#pragma unroll
+      for (int k = 0; k < 15; ++k)
+#pragma unroll
+        for (int r = k + 1; r < 16; ++r) cfms(x[r], B[r + k * TI_LD], x[k]);
+    } else {
+#pragma unroll
+      for (int k = 15; k >= 0; --k) {
+        x[k] = cmul(x[k], rcps[o16 + k]);
+#pragma unroll
+        for (int r = 0; r < k; ++r) cfms(x[r], B[r + k * TI_LD], x[k]);
+      }
+    }
+    __syncwarp(0x0000ffffu);          // every lane has read its triangle of the block
+    T *C = D + o16 + (o16 + l) * TI_LD;
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+      if (w < 4 ? r > l : r <= l) C[r] = x[r];
+  }
+  __syncthreads();
+  // entries of the two inverses: L^-1 with its unit diagonal and zeros above, U^-1 with zeros below
+  auto xl = [&](int r, int c) { return r > c ? D[r + c * TI_LD] : (r == c ? one : zero); };
+  auto xu = [&](int r, int c) { return r <= c ? D[r + c * TI_LD] : zero; };
+  if (jb > 16) {
+    // 16 -> 32, blocks at o = 0 and 32: warp w takes product w >> 1 (L at 0, 32, then U at 0, 32),
+    // columns 8 (w & 1).. + 7; lane: row lane & 15, columns 4 (lane >> 4) + q
+    const bool up = w >= 4;
+    const int o = 32 * ((w >> 1) & 1), i = lane & 15, j0 = 8 * (w & 1) + 4 * (lane >> 4);
+    T v[4], y[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = y[q] = zero;
+    if (o + 16 < jb) {
+#pragma unroll 4
+      for (int k = 0; k < 16; ++k) {
+        const T d = up ? D[(o + i) + (o + 16 + k) * TI_LD] : D[(o + 16 + i) + (o + k) * TI_LD];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          cfma(v[q], d, up ? xu(o + 16 + k, o + 16 + j0 + q) : xl(o + k, o + j0 + q));
+      }
+    }
+    T *P = up ? D + o + (o + 16) * TI_LD : D + o + 16 + o * TI_LD;     // the off-diagonal block
     __syncthreads();
-    for (int i = j + 1 + t; i < n; i += nt) {
-      T s = tmp[i];
-      for (int k = j + 1; k < i; ++k) cfma(s, D[i + k * NB], tmp[k]);
-      D[i + j * NB] = cneg(s);
+    if (o + 16 < jb) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) P[i + (j0 + q) * TI_LD] = v[q];
+    }
+    __syncthreads();
+    if (o + 16 < jb) {
+#pragma unroll 4
+      for (int k = 0; k < 16; ++k) {
+        const T x = up ? xu(o + i, o + k) : xl(o + 16 + i, o + 16 + k);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cfms(y[q], x, P[k + (j0 + q) * TI_LD]);
+      }
+    }
+    __syncthreads();
+    if (o + 16 < jb) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) P[i + (j0 + q) * TI_LD] = y[q];
     }
     __syncthreads();
   }
-  for (int j = 0; j < n; ++j) {
-    if (t == 0) { T d = crcp(D[j + j * NB]); D[j + j * NB] = d; s_d = d; }
-    for (int i = t; i < j; i += nt) tmp[i] = D[i + j * NB];
-    __syncthreads();
-    const T d = s_d;
-    for (int i = t; i < j; i += nt) {
-      T s = czero<T>();
-      for (int k = i; k < j; ++k) cfma(s, D[i + k * NB], tmp[k]);
-      D[i + j * NB] = cneg(cmul(d, s));
+  if (jb > 32) {
+    // 32 -> 64: warps 0..3 L, 4..7 U; warp columns 8 (w & 3) + q, lane = row.  X00(k, j) = 0 for
+    // k < j and Y11(k, j) = 0 for k > j: the inner products take the triangular half of the work
+    const bool up = w >= 4;
+    const int i = lane, j0 = 8 * (w & 3);
+    T v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = zero;
+    T *P = up ? D + 32 * TI_LD : D + 32;
+    const int k0 = up ? 0 : j0, k1 = up ? j0 + 8 : 32;
+#pragma unroll 2
+    for (int k = k0; k < k1; ++k) {
+      const T d = P[i + k * TI_LD];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) cfma(v[q], d, up ? xu(32 + k, 32 + j0 + q) : xl(k, j0 + q));
     }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      P[i + (j0 + q) * TI_LD] = v[q];
+      v[q] = zero;
+    }
+    __syncwarp();                     // a warp's product columns are read by that warp only
+#pragma unroll 2
+    for (int k = 0; k < 32; ++k) {
+      const T x = up ? xu(i, k) : xl(32 + i, 32 + k);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) cfms(v[q], x, P[k + (j0 + q) * TI_LD]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) P[i + (j0 + q) * TI_LD] = v[q];
     __syncthreads();
   }
   const size_t off = ((size_t)b * nsteps + J / NB) * NB * NB;
-  for (int e = t; e < NB * NB; e += nt) {
-    int i = e % NB, k = e / NB;
-    T lv = czero<T>(), uv = czero<T>();
-    if (i < n && k < n) {
-      if (i > k) lv = D[i + k * NB];
-      else if (i == k) lv = cx<T>::make(1, 0);
-      if (i <= k) uv = D[i + k * NB];
-    }
-    Linv[off + e] = lv;
-    Uinv[off + e] = uv;
+#pragma unroll 4
+  for (int e = t; e < NB * NB; e += 256) {
+    const int i = e % NB, k = e / NB;
+    const bool in = i < jb && k < jb;
+    Linv[off + e] = in ? xl(i, k) : zero;
+    Uinv[off + e] = in ? xu(i, k) : zero;
   }
 }
 
@@ -1142,30 +1266,30 @@ k_trisolve_smem(const T *M, size_t strideM, int N, int NB, int nsteps, const T *
 // ---------------------------------------------------------------------------
 // host drivers
 // ---------------------------------------------------------------------------
+template <typename T, int RPT, int SW, int NTMAX>
+static cudaError_t launch_panel_as(T *M, const LUBatch &lb, int J, int jb, cudaStream_t st) {
+  const int rows = lb.N - J;
+  const int nt = std::max(128, ((rows + RPT - 1) / RPT + 31) / 32 * 32);
+  const size_t dyn = sizeof(T) * (size_t)64 * 2 * SW;
+  smem_limit(k_panel<T, RPT, SW, NTMAX>, (int)dyn);
+  k_panel<T, RPT, SW, NTMAX><<<lb.batch, nt, dyn, st>>>(M, lb.strideM, lb.N, J, jb, lb.ipiv, lb.info);
+  return ADGA_LAUNCH_CHECK();
+}
+
 template <typename T>
 static cudaError_t launch_panel(T *M, const LUBatch &lb, int J, int jb, cudaStream_t st) {
   const int rows = lb.N - J;
-  auto nthreads = [&](int rpt) { int n = ((rows + rpt - 1) / rpt + 31) / 32 * 32; return n < 32 ? 32 : n; };
-  const size_t dyn = sizeof(T) * (size_t)MAXNB * 2 * SWD;
-  smem_limit(k_panel<T, 1>, 96 * 1024);
-  smem_limit(k_panel<T, 2>, 96 * 1024);
-  smem_limit(k_panel<T, 4>, 96 * 1024);
-  smem_limit(k_panel<T, 8>, 96 * 1024);
-  // fewer, fuller threads per CTA: more matrices resident per SM and cheaper
-  // block-wide pivot reductions (FP32 rows cost half the registers of FP64)
-  const bool f32 = sizeof(T) == sizeof(z32);
-  if (rows <= (f32 ? 0 : 1024)) {
-    k_panel<T, 1><<<lb.batch, nthreads(1), dyn, st>>>(M, lb.strideM, lb.N, J, jb, lb.ipiv, lb.info);
-  } else if (rows <= (f32 ? 0 : 1280)) {
-    k_panel<T, 2><<<lb.batch, nthreads(2), dyn, st>>>(M, lb.strideM, lb.N, J, jb, lb.ipiv, lb.info);
-  } else if (rows <= 2048) {
-    k_panel<T, 4><<<lb.batch, nthreads(4), dyn, st>>>(M, lb.strideM, lb.N, J, jb, lb.ipiv, lb.info);
-  } else if (rows <= 4096) {
-    k_panel<T, 8><<<lb.batch, nthreads(8), dyn, st>>>(M, lb.strideM, lb.N, J, jb, lb.ipiv, lb.info);
-  } else {
-    return cudaErrorInvalidValue;   // N > 4096 is not supported
-  }
-  return ADGA_LAUNCH_CHECK();
+  // rows x SW complex values fill the register file at 512 x 16, 1024 x 8, 2048 x 4 and 4096 x 2; wider
+  // sub-panels halve the passes over the rest of the panel, spilled ones cost more than they save
+  // (one 64-column panel, us, as listed / with the next wider or narrower form: 1016 rows 255 / 301,
+  // 1080 rows 330 / 395, 1500 rows 418 / 428, 2000 rows 543 / 998, 4000 rows 2666 / 3839)
+  if (rows <= 512) return launch_panel_as<T, 1, 16, 512>(M, lb, J, jb, st);
+  if (rows <= 1024) return launch_panel_as<T, 2, 8, 512>(M, lb, J, jb, st);
+  if (rows <= 1280) return launch_panel_as<T, 2, 4, 640>(M, lb, J, jb, st);
+  if (rows <= 1536) return launch_panel_as<T, 2, 4, 768>(M, lb, J, jb, st);
+  if (rows <= 2048) return launch_panel_as<T, 4, 4, 512>(M, lb, J, jb, st);
+  if (rows <= 4096) return launch_panel_as<T, 8, 2, 512>(M, lb, J, jb, st);
+  return cudaErrorInvalidValue;   // N > 4096 is not supported
 }
 
 cudaError_t lu_trail_z64(z64 *M, const LUBatch &lb, int J, int jb, cudaStream_t st);
@@ -1278,10 +1402,10 @@ cudaError_t lu_factor_groups(z32 *M, const LUBatch &lb, const GroupOps &ops, cud
 template <typename T>
 cudaError_t lu_step(T *M, const LUBatch &lb, int s, bool apply_left, trail_fn trail, void *trail_ctx,
                     cudaStream_t st, TrailTiming *tt, bool nopiv) {
-  if (lb.NB > 64 || lb.NB % SWD) return cudaErrorInvalidValue;   // k_swap_trsm covers NB <= 64
+  if (lb.NB > 64 || lb.NB % 8) return cudaErrorInvalidValue;   // the step kernels cover NB <= 64
   const int nsteps = lb.nsteps();
   cudaError_t e;
-  const size_t sm_tri = sizeof(T) * ((size_t)lb.NB * lb.NB + lb.NB);
+  const size_t sm_tri = sizeof(T) * 64 * TI_LD;
   const size_t sm_trsm = sizeof(typename TrsmOp<T>::L) * 64 * 64 + sizeof(typename TrsmOp<T>::X) * TW * TS_LD;
   smem_limit(k_triinv<T>, 200 * 1024);
   smem_limit(k_swap_trsm<T>, 200 * 1024);

@@ -1,0 +1,48 @@
+"""The FP64 LU with partial pivoting at the sizes where its kernels change
+shape: one step and several (64 columns each), sub-panels of 16 and 8 columns,
+one to eight rows per thread (512, 1024, 1536, 2048 rows), ragged last steps."""
+import numpy as np
+import pytest
+
+from adga_b200 import inverse_matrix
+
+SIZES = [1, 2, 7, 8, 15, 16, 17, 31, 33, 40, 63, 64, 65, 79, 80, 128, 129, 357, 511, 512, 513, 577, 1024, 1025, 1089,
+         1537, 2049]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", SIZES)
+def test_inverse_residual(n):
+    """Backward-stable elimination: |X A - 1|_2 <= c n eps cond(A) with a
+    modest growth factor in c (32)."""
+    rng = np.random.default_rng(n)
+    A = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / np.sqrt(2 * n)
+    X, ierr, _ = inverse_matrix(A)
+    assert ierr == 0
+    s = np.linalg.svd(A, compute_uv=False)
+    tol = 32 * n * np.finfo(float).eps * s[0] / s[-1]
+    assert np.linalg.norm(X @ A - np.eye(n), 2) <= tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", SIZES)
+def test_inverse_of_signed_permutation_is_exact(n):
+    """Every pivot is far from the diagonal and every operation is exact."""
+    rng = np.random.default_rng(1000 + n)
+    A = np.zeros((n, n), dtype=complex)
+    A[np.arange(n), rng.permutation(n)] = rng.choice([1, -1, 1j, -1j], n) * 2.0 ** rng.integers(-40, 40, n)
+    X, ierr, _ = inverse_matrix(A)
+    assert ierr == 0
+    want = np.zeros_like(A)
+    r, c = np.nonzero(A)
+    want[c, r] = A[r, c].conj() / np.abs(A[r, c]) ** 2
+    assert np.array_equal(X, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,col", [(1, 0), (40, 17), (64, 63), (65, 64), (200, 130), (600, 5), (1030, 1029)])
+def test_zero_column_is_reported(n, col):
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    A[:, col] = 0.0
+    assert inverse_matrix(A)[1] == col + 1
