@@ -14,16 +14,13 @@
 
 using namespace zg;
 
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, 3)
 k_tan_rhs(int N, int R, int npts, int ch, const z64 *__restrict__ XS, const z64 *__restrict__ Frow,
           const z64 *__restrict__ XD, const z64 *__restrict__ Fdot, const z64 *__restrict__ dB, z64 *out) {
   extern __shared__ __align__(16) z64 zg_smem[];
-  z64 *As = zg_smem, *Bs = zg_smem + STAGES * BK * BM;
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
   const int rows = npts * R;
   const int r0 = blockIdx.y * BM, c0 = blockIdx.x * BN;
   const size_t per = (size_t)R * N;
-  z64 acc[TM][TN], acc2[TM][TN];
   auto la_of = [&](const z64 *A) {
     return [=](int r, int k) -> const z64 * {
       const int row = r0 + r;
@@ -38,29 +35,26 @@ k_tan_rhs(int N, int R, int npts, int ch, const z64 *__restrict__ XS, const z64 
       return (k < N && cl < N) ? B + (size_t)k * N + cl : nullptr;
     };
   };
+  Acc acc;
+  clear(acc);
+  if (XS) mainloop<true, true>(acc, zg_smem, N, rows - r0, N - c0, la_of(XS), lb_of(Frow), Frow);
+  if (XD && Fdot) mainloop<true, true>(acc, zg_smem, N, rows - r0, N - c0, la_of(XD), lb_of(Fdot), Fdot);
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = acc2[i][j] = make_double2(0.0, 0.0);
-  if (XS) mainloop<true, true>(acc, As, Bs, N, la_of(XS), lb_of(Frow), Frow);
-  if (XD && Fdot) {
-    __syncthreads();
-    mainloop<true, true>(acc2, As, Bs, N, la_of(XD), lb_of(Fdot), Fdot);
-  }
-#pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int row = r0 + tx + 16 * i;
+  for (int i = 0; i < 4; ++i) {
+    const int row = r0 + row_of(i);
     if (row >= rows) continue;
     const int p = row / R, i1 = row % R;
     const size_t m = (size_t)(2 * p + ch);
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int cl = c0 + ty + 16 * j;
-      if (cl >= N) continue;
-      z64 v = cadd(acc[i][j], acc2[i][j]);
-      if (dB) v = cadd(v, dB[i1 + (size_t)cl * R]);
-      out[m * per + (size_t)i1 * N + cl] = v;
-    }
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int cl = c0 + col_of(j, e);
+        if (cl >= N) continue;
+        z64 v = make_double2(acc.re[i][j][e], acc.im[i][j][e]);
+        if (dB) v = cadd(v, dB[i1 + (size_t)cl * R]);
+        out[m * per + (size_t)i1 * N + cl] = v;
+      }
   }
 }
 

@@ -1,4 +1,4 @@
-// Complex FP64 GEMMs on the CUDA cores built on zgemm.cuh:
+// Complex FP64 GEMMs built on zgemm.cuh:
 //   * k_trail_z64  -- the FP64 LU trailing update A22 -= L21 U12 (batched);
 //   * k_resid_z64  -- the refinement residual r = B - X + (X D) F~ of the
 //                     mixed path (rows = points x ndim2, K = N, F~ shared).
@@ -8,11 +8,12 @@
 
 using namespace zg;
 
-__global__ void __launch_bounds__(NT)
+// Bound by the FP64 rate (8 flops per complex product; the C read and write takes two fifths of
+// that time).  C's lines are prefetched into L2 before the products, and the difference is taken
+// at the end: the sum over k is rounded at its own size and C once.
+__global__ void __launch_bounds__(NT, 3)
 k_trail_z64(z64 *M, size_t strideM, int N, int ncols, int J, int jb) {
   extern __shared__ __align__(16) z64 zg_smem[];
-  z64 *As = zg_smem, *Bs = zg_smem + STAGES * BK * BM;
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
   z64 *A = M + (size_t)blockIdx.z * strideM;
   const int r0 = J + jb + blockIdx.y * BM, c0 = J + jb + blockIdx.x * BN;
   auto la = [&](int r, int k) -> const z64 * {
@@ -23,23 +24,35 @@ k_trail_z64(z64 *M, size_t strideM, int N, int ncols, int J, int jb) {
     const int cc = c0 + c;
     return (k < jb && cc < ncols) ? A + (J + k) + (size_t)cc * N : nullptr;
   };
-  z64 acc[TM][TN];
-  mainloop<false, false>(acc, As, Bs, jb, la, lb, A);
-  z64 cv[TM][TN];
+  {
+    const int c = c0 + (threadIdx.x >> 1), r = r0 + 32 * (threadIdx.x & 1);
 #pragma unroll
-  for (int j = 0; j < TN; ++j)
+    for (int q = 0; q < 4; ++q)
+      if (c < ncols && r + 8 * q < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(A + r + 8 * q + (size_t)c * N));
+  }
+  Acc acc;
+  clear(acc);
+  mainloop<false, false>(acc, zg_smem, jb, N - r0, ncols - c0, la, lb, A);
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const int r = r0 + tx + 16 * i, c = c0 + ty + 16 * j;
-      cv[i][j] = (r < N && c < ncols) ? A[r + (size_t)c * N] : make_double2(0.0, 0.0);
-    }
+  for (int i = 0; i < 4; ++i) {
+    const int r = r0 + row_of(i);
+    z64 cv[4][2];
 #pragma unroll
-  for (int j = 0; j < TN; ++j)
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const int r = r0 + tx + 16 * i, c = c0 + ty + 16 * j;
-      if (r < N && c < ncols) A[r + (size_t)c * N] = csub(cv[i][j], acc[i][j]);
-    }
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + col_of(j, e);
+        cv[j][e] = (r < N && c < ncols) ? A[r + (size_t)c * N] : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + col_of(j, e);
+        if (r < N && c < ncols)
+          A[r + (size_t)c * N] = make_double2(cv[j][e].x - acc.re[i][j][e], cv[j][e].y - acc.im[i][j][e]);
+      }
+  }
 }
 
 cudaError_t lu_trail_z64(z64 *M, const LUBatch &lb, int J, int jb, cudaStream_t st) {
@@ -53,13 +66,11 @@ cudaError_t lu_trail_z64(z64 *M, const LUBatch &lb, int J, int jb, cudaStream_t 
 
 // rows (p, i1) of channel ch, columns c:
 //   V(p,i1,c) = fp32( opg(i1,c) - X(p,i1,c) + sum_m XD(p,i1,m) F~(m,c) )
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, 3)
 k_resid_z64(int N, int R, int npts, int ch, const z64 *__restrict__ XD, const z64 *__restrict__ X,
             const z64 *__restrict__ Frow, const z64 *__restrict__ opg, z32 *V, const z64 *__restrict__ extra,
             unsigned long long *rnorm, const z64 *__restrict__ Bpt) {
   extern __shared__ __align__(16) z64 zg_smem[];
-  z64 *As = zg_smem, *Bs = zg_smem + STAGES * BK * BM;
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
   const int rows = npts * R;
   const int r0 = blockIdx.y * BM, c0 = blockIdx.x * BN;
   const size_t per = (size_t)R * N;
@@ -73,29 +84,33 @@ k_resid_z64(int N, int R, int npts, int ch, const z64 *__restrict__ XD, const z6
     const int cl = c0 + c;
     return (k < N && cl < N) ? Frow + (size_t)k * N + cl : nullptr;
   };
-  z64 acc[TM][TN];
-  mainloop<true, true>(acc, As, Bs, N, la, lb, Frow);
+  Acc acc;
+  clear(acc);
+  mainloop<true, true>(acc, zg_smem, N, rows - r0, N - c0, la, lb, Frow);
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int row = r0 + tx + 16 * i;
+  for (int i = 0; i < 4; ++i) {
+    const int row = r0 + row_of(i);
     const int p = row / R, i1 = row % R;
     const size_t m = (size_t)(2 * p + ch);
     double rmax = 0.0;
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int cl = c0 + ty + 16 * j;
-      if (row >= rows || cl >= N) continue;
-      // right-hand side: (1+gamma^w) shared by the slice, or per point (tangent solves)
-      const z64 b = Bpt ? Bpt[m * per + (size_t)i1 * N + cl] : opg[i1 + (size_t)cl * R];
-      const z64 x = X[m * per + (size_t)i1 * N + cl];
-      z64 r = make_double2(b.x - x.x + acc[i][j].x, b.y - x.y + acc[i][j].y);
-      if (extra) r = cadd(r, extra[(size_t)p * per + (size_t)i1 * N + cl]);   // V(q) term (density)
-      V[m * per + (size_t)i1 * N + cl] = to32(r);
-      rmax = fmax(rmax, fabs(r.x) + fabs(r.y));
-    }
-    // max |re| + |im| of the FP64 residual per matrix (lanes t and t + 16 share their rows)
-    rmax = fmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, 16));
-    if (rnorm && ty % 2 == 0 && row < rows && rmax > 0.0)
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int cl = c0 + col_of(j, e);
+        if (row >= rows || cl >= N) continue;
+        // right-hand side: (1+gamma^w) shared by the slice, or per point (tangent solves)
+        const z64 b = Bpt ? Bpt[m * per + (size_t)i1 * N + cl] : opg[i1 + (size_t)cl * R];
+        const z64 x = X[m * per + (size_t)i1 * N + cl];
+        z64 r = make_double2(b.x - x.x + acc.re[i][j][e], b.y - x.y + acc.im[i][j][e]);
+        if (extra) r = cadd(r, extra[(size_t)p * per + (size_t)i1 * N + cl]);   // V(q) term (density)
+        V[m * per + (size_t)i1 * N + cl] = to32(r);
+        rmax = fmax(rmax, fabs(r.x) + fabs(r.y));
+      }
+    // max |re| + |im| of the FP64 residual per matrix (four lanes share a row)
+    rmax = fmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, 1));
+    rmax = fmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, 2));
+    if (rnorm && threadIdx.x % 4 == 0 && row < rows && rmax > 0.0)
       atomicMax(rnorm + (size_t)(2 * p + ch), (unsigned long long)__double_as_longlong(rmax));
   }
 }
