@@ -11,7 +11,7 @@
 struct DftView {
   const z64 *ghat;               // null: the direct k-sum kernels only
   int m[3];
-  int min_points;                // batches with fewer points use the direct kernels
+  int min_points, eom_min_points;   // batches with fewer points use the direct kernels
   const int *qlin;               // (nqp)
   const double2 *twk[3], *twm[3];
   z64 *a, *b;

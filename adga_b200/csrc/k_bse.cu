@@ -441,7 +441,7 @@ k_eom_dyn(DevCtx c, int iwb, const int *__restrict__ qidx, int npts, const z64 *
 cudaError_t launch_eom_dynamic(const DevCtx &c, int iwb, const int *qidx, int npts,
                                const z64 *mtot, z64 *sigma_nl, cudaStream_t st) {
   if (npts <= 0) return cudaSuccess;
-  if (c.dft.ghat && npts >= c.dft.min_points)
+  if (c.dft.ghat && npts >= c.dft.eom_min_points)
     return launch_eom_dft(c, iwb, qidx, npts, mtot, c.dft.ghat, sigma_nl, st);
   dim3 grid(cdiv_u(c.nkp_eom, 128), c.iwf);
   switch (c.nd) {

@@ -5,6 +5,8 @@ k - q kernels and the oracle.
 ADGA_DFT_MIN_POINTS=1 forces the transform for every batch, ADGA_BUBBLE=direct
 keeps the direct kernels; both are read when a handle is created.
 """
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -107,3 +109,23 @@ def test_transform_tangents_match_direct(par):
             lad.close()
     for k in OUT_KEYS:
         assert rel_err(res[0][k], res[1][k]) < 1e-12, (k, rel_err(res[0][k], res[1][k]))
+
+
+@pytest.mark.parametrize("name,nk,nq", [("t1", (10, 10, 11), (5, 5, 1)), ("t2", (12, 12, 9), (6, 3, 3)),
+                                        ("t3", (8, 8, 9), (4, 4, 3)), ("t5", (6, 6, 7), (3, 3, 7))])
+@pytest.mark.parametrize("points", [1, 3, 16, 17])
+def test_few_points_match_transform(name, nk, nq, points):
+    """The direct sums for up to 16 points (k-points shared by a cluster of
+    blocks, ragged last chunk) and the gather kernel beyond, both against the
+    transform: the same sum in another order (1e-12, as above)."""
+    p = synth.make_problem(dataclasses.replace(synth.SPECS[name], nk=nk, nq=nq))
+    got = []
+    for settings in (TRANSFORM, DIRECT):
+        lad = make_ladder(p, settings)
+        try:
+            lad.ladder_run(3, 2 + points, "fp64")
+            got.append(lad.get_outputs())
+        finally:
+            lad.close()
+    for k in ("bubble_nl", "chi_qw_dens", "chi_qw_magn", "sigma_nl"):
+        assert rel_err(got[1][k], got[0][k]) < 1e-12, (k, rel_err(got[1][k], got[0][k]))
