@@ -1219,9 +1219,13 @@ static int run_batch(adga_handle *h, int iwb, int np, int off, int prec, int *st
     CK(launch_bse_build<z64>(c, np, chi0q, h->c0inv, h->Frow_d, h->Frow_m, h->opg_d, h->opg_m, T,
                              strideM, h->gq, h->qidx_d, st));
     cudaEventRecord(ev[2], st);
-    // tangents solve with L as well: keep the interchanges on the left columns
-    CK(factor_batch<z64>(h, T, lb, h->tan_on, false, &tt));
-    CK(lu_backsolve<z64>(T, lb, T + N * N, strideM, (int)N, (int)R, st));
+    if (!h->tan_on && lu_small_supported((int)N, (int)R)) {
+      CK(lu_small_solve(T, strideM, (int)N, (int)R, 2 * np, h->info, st));
+    } else {
+      // tangents solve with L as well: keep the interchanges on the left columns
+      CK(factor_batch<z64>(h, T, lb, h->tan_on, false, &tt));
+      CK(lu_backsolve<z64>(T, lb, T + N * N, strideM, (int)N, (int)R, st));
+    }
     X = T + N * N; sp = 2 * strideM; sc = strideM;
   } else {
     z32 *T = (z32 *)h->Tm;
@@ -1990,8 +1994,12 @@ extern "C" int adga_inverse_matrix_z(adga_z *M, int n, int *ierr, char *erstr) {
     int info = 0;
     cudaError_t e = cudaMemcpyAsync(T, aug.data(), sizeof(z64) * strideM, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(inf, 0, sizeof(int), st);
-    if (e == cudaSuccess) e = lu_factor<z64>(T, lb, false, nullptr, nullptr, st);
-    if (e == cudaSuccess) e = lu_backsolve<z64>(T, lb, T + (size_t)n * n, strideM, n, n, st);
+    if (lu_small_supported(n, n)) {
+      if (e == cudaSuccess) e = lu_small_solve(T, strideM, n, n, 1, inf, st);
+    } else {
+      if (e == cudaSuccess) e = lu_factor<z64>(T, lb, false, nullptr, nullptr, st);
+      if (e == cudaSuccess) e = lu_backsolve<z64>(T, lb, T + (size_t)n * n, strideM, n, n, st);
+    }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&info, inf, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(M, T + (size_t)n * n, sizeof(z64) * n * n, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -96,6 +96,11 @@ cudaError_t lu_backsolve(const T *M, const LUBatch &lb, T *C, size_t strideC, in
 template <typename T>
 cudaError_t lu_fwdsolve_ws(const T *M, const LUBatch &lb, T *V, size_t strideV, int ldv, int R,
                            T *work, cudaStream_t st);
+// k_lu_small.cu: factorisation and back substitution of systems that fit in shared memory; the
+// solutions replace the right-hand sides (columns N.. of the matrix), the rest of it is left as it
+// was, and no factors, pivots or block inverses are kept
+bool lu_small_supported(int N, int R);
+cudaError_t lu_small_solve(z64 *M, size_t strideM, int N, int R, int batch, int *info, cudaStream_t st);
 // the factorization's row permutation, from ipiv, into perm[batch][N]
 cudaError_t lu_build_perm(const LUBatch &lb, int *perm, cudaStream_t st);
 // streaming solves (k_trsv.cu): NB = 64, R <= 25; the forward one needs lb.perm and work
