@@ -9,86 +9,238 @@
 //   * eom    -- Sigma(k, nu) += m_tot G(k-q, nu-w) over a batch of points
 //               (src/eom_module.f90:209-230), one owner thread per (k, nu).
 #include "ctx.cuh"
+#include "zgemm.cuh"
 #include <algorithm>
 #include <type_traits>
 
 // ---------------------------------------------------------------------------
-// build: one block per (column tile of A^T rows c, channel, point).
-// T(c, r) = delta(c, r) - sum_i3 sw_nu(i1, i3) F~(i3 + nu*nd2, c), r = i1 + nu*nd2
-// sw_nu = chi0q(:,:,nu) diag(chi0_loc^-1(nu)) - 1
+// build: T(c, r) = delta(c, r) - sum_i3 sw_nu(i1, i3) F~(i3 + nu*nd2, c), r = i1 + nu*nd2,
+// sw_nu = chi0q(:,:,nu) diag(chi0_loc^-1(nu)) - 1, and gamma^q_d = sum_nu sw_nu F~_d(nu block).
 // ---------------------------------------------------------------------------
-template <typename T, int ND2>
-__global__ void __launch_bounds__(128)
-k_bse_build(DevCtx c, const z64 *__restrict__ chi0q, const z64 *__restrict__ c0inv,
-            const z64 *__restrict__ Frow_d, const z64 *__restrict__ Frow_m,
-            const z64 *__restrict__ opg_d, const z64 *__restrict__ opg_m, T *Tm, size_t strideM,
-            z64 *gammaqd, const int *__restrict__ qidx) {
-  __shared__ z64 sw[ND2 * ND2];
-  __shared__ z64 sv[ND2 * ND2];   // 2 beta^-2 chi0^q(nu) v(q), density channel with V(q)
-  const int N = c.N;
-  const int cc = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ch = blockIdx.y, p = blockIdx.z;
-  const z64 *F = ch == 0 ? Frow_d : Frow_m;
-  const z64 *opg = ch == 0 ? opg_d : opg_m;
+// One orbital: element by element.  A warp takes 32 columns and every eighth nu, so that the
+// frequencies are not one serial chain per column; gamma^q_d adds the warps' parts in their order.
+// (A thread per column walking all nu took 18 us a channel on N = 40 and 65 us on N = 160 with 216
+// points; this kernel, both channels: 5.4 and 47 us.)
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_bse_build_1(DevCtx c, const z64 *__restrict__ chi0q, const z64 *__restrict__ c0inv,
+              const z64 *__restrict__ Frow_d, const z64 *__restrict__ Frow_m, const z64 *__restrict__ opg_d,
+              const z64 *__restrict__ opg_m, T *Tm, size_t strideM, z64 *gammaqd, const int *__restrict__ qidx) {
+  __shared__ z64 part[8][32];
+  const int N = c.N, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cc = blockIdx.x * 32 + lane, ch = blockIdx.y, p = blockIdx.z;
+  const z64 *F = ch == 0 ? Frow_d : Frow_m, *opg = ch == 0 ? opg_d : opg_m, *c0 = chi0q + (size_t)p * N;
   T *Tp = Tm + (size_t)(2 * p + ch) * strideM;
-  const z64 *c0 = chi0q + (size_t)p * ND2 * ND2 * 2 * c.iwf;
-  z64 gq[ND2];
-#pragma unroll
-  for (int a = 0; a < ND2; ++a) gq[a] = make_double2(0.0, 0.0);
-  const bool vterm = c.vq && ch == 0;
-  const z64 *vq = vterm ? c.vq + (size_t)qidx[p] * ND2 * ND2 : nullptr;
-  z64 og[ND2];                      // (1 + gamma^w_d)(:, cc)
-  if (vterm && cc < N)
-#pragma unroll
-    for (int i3 = 0; i3 < ND2; ++i3) og[i3] = opg_d[i3 + (size_t)cc * ND2];
-  for (int dum = 0; dum < 2 * c.iwf; ++dum) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < ND2 * ND2; e += blockDim.x) {
-      int i1 = e % ND2, i3 = e / ND2;
-      z64 v = cmul(c0[(size_t)dum * ND2 * ND2 + e], c0inv[dum * ND2 + i3]);
-      if (i1 == i3) v.x -= 1.0;
-      sw[e] = v;                       // sw(i1, i3) at i1 + i3*nd2
-      if (vterm) {                     // src/main.F90:710-719
-        z64 t = make_double2(0.0, 0.0);
-        for (int m = 0; m < ND2; ++m) cfma(t, c0[(size_t)dum * ND2 * ND2 + i1 + m * ND2], vq[m + i3 * ND2]);
-        const double f = 2.0 / (c.beta * c.beta);
-        sv[e] = make_double2(f * t.x, f * t.y);
-      }
-    }
-    __syncthreads();
-    if (cc < N) {
-      z64 f[ND2];
-#pragma unroll
-      for (int i3 = 0; i3 < ND2; ++i3) f[i3] = F[(size_t)(i3 + dum * ND2) * N + cc];
-#pragma unroll
-      for (int i1 = 0; i1 < ND2; ++i1) {
-        z64 w = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int i3 = 0; i3 < ND2; ++i3) cfma(w, sw[i1 + i3 * ND2], f[i3]);
-        int r = i1 + dum * ND2;
-        z64 t = make_double2(-w.x, -w.y);
-        if (vterm)
-#pragma unroll
-          for (int i3 = 0; i3 < ND2; ++i3) cfms(t, sv[i1 + i3 * ND2], og[i3]);
-        if (r == cc) t.x += 1.0;
-        Tp[cc + (size_t)r * N] = from64<T>(t);
-        if (ch == 0) gq[i1] = cadd(gq[i1], w);
-      }
-    }
+  const bool act = cc < N;
+  z64 og = act ? opg[cc] : czero<z64>(), sv = czero<z64>();
+  if (c.vq && ch == 0) sv = cscale(c.vq[qidx[p]], 2.0 / (c.beta * c.beta));    // src/main.F90:710-719
+  z64 gq = czero<z64>();
+#pragma unroll 4
+  for (int nu = w; nu < N; nu += 8) {
+    const z64 q = c0[nu];
+    z64 sw = cmul(q, c0inv[nu]);
+    sw.x -= 1.0;
+    const z64 g = act ? cmul(sw, F[(size_t)nu * N + cc]) : czero<z64>();
+    gq = cadd(gq, g);
+    z64 t = cneg(g);
+    if (c.vq && ch == 0) cfms(t, cmul(q, sv), og);
+    if (nu == cc) t.x += 1.0;
+    if (act) Tp[cc + (size_t)nu * N] = from64<T>(t);
   }
-  if (cc < N) {
-#pragma unroll
-    for (int i1 = 0; i1 < ND2; ++i1) Tp[cc + (size_t)(N + i1) * N] = from64<T>(opg[i1 + (size_t)cc * ND2]);
+  part[w][lane] = gq;
+  __syncthreads();
+  if (w == 0 && act) {
+    Tp[cc + (size_t)N * N] = from64<T>(og);
     if (ch == 0 && gammaqd) {
-      z64 *g = gammaqd + (size_t)p * ND2 * N;
-#pragma unroll
-      for (int i1 = 0; i1 < ND2; ++i1) g[i1 + (size_t)cc * ND2] = gq[i1];
+      for (int v = 1; v < 8; ++v) gq = cadd(gq, part[v][lane]);
+      gammaqd[(size_t)p * N + cc] = gq;
     }
   }
 }
 
-// Fast build (no V(q) term): one block per (128-column tile, P points) of one
-// channel.  A thread owns one column c of T; the F~ rows of each nu block are
+// Four and five orbitals, and the density channel with V(q): per nu a product of the batch's sw rows (npts nd2 x nd2) with the nd2 x N block of F~
+// on the FP64 tensor cores (m8n8k4, complex as four real products).  A CTA owns 32 rows (p, i1) and 64
+// columns and walks nu: F~'s block of the next nu arrives by cp.async while sw of the next nu is formed
+// from chi0^q into the other half of the stage; K = nd2 is padded with zeros to a multiple of four (4, 12,
+// 16, 28).  Bound by the FP64 rate (padding included) with F~ read from L2 and T written once.  GQ (the
+// density channel) keeps gamma^q_d's sum over nu in registers; with V(q) the term
+// 2 beta^-2 chi0^q(nu) v(q) (1+gamma^w_d) (src/main.F90:710-719) is a second product with a resident
+// operand, after gamma^q_d has taken the first.
+// A thread per column with all products on the CUDA cores took 8.8 ms (both channels, 216 points,
+// N = 1000, 25 components; this kernel 4.45 ms) and 0.81 ms (both, 216 points, N = 486, with V(q); this
+// kernel for the density channel 0.62 ms, the magnetic one as without V(q) 0.25 ms).
+template <int ND2> struct BuildTile {
+  static constexpr int KP = (ND2 + 3) / 4 * 4;
+  static constexpr int LDA = KP % 8 == 4 ? KP : KP + 4, LDB = 66;      // conflict-free fragment reads
+  static constexpr int A_ELEMS = 32 * LDA, B_ELEMS = KP * LDB;
+  static constexpr int smem(bool vterm) {
+    return (int)sizeof(z64) * (2 * (A_ELEMS + B_ELEMS) + (vterm ? 2 * A_ELEMS + B_ELEMS : 0));
+  }
+};
+
+template <typename TW, int ND2, bool GQ>
+__global__ void __launch_bounds__(128, 2)
+k_bse_build(DevCtx c, int npts, int ch, const z64 *__restrict__ chi0q, const z64 *__restrict__ c0inv,
+            const z64 *__restrict__ F, const z64 *__restrict__ opg, TW *Tm, size_t strideM, z64 *gammaqd,
+            const int *__restrict__ qidx) {
+  typedef BuildTile<ND2> L;
+  constexpr int KP = L::KP, NE = (32 * ND2 + 127) / 128;
+  extern __shared__ __align__(16) z64 bse_smem[];
+  z64 *As = bse_smem, *Bs = As + 2 * L::A_ELEMS, *Vs = Bs + 2 * L::B_ELEMS, *Og = Vs + 2 * L::A_ELEMS;
+  const int N = c.N, nnu = 2 * c.iwf, t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int c0 = blockIdx.x * 64, m0 = blockIdx.y * 32, rows = npts * ND2;
+  const bool vterm = GQ && c.vq;
+  for (int e = t; e < L::smem(vterm) / (int)sizeof(z64); e += 128) bse_smem[e] = czero<z64>();   // the padding
+  __syncthreads();
+  auto stage_f = [&](int nu, int buf) {
+    for (int e = t; e < ND2 * 64; e += 128) {
+      const int k = e >> 6, col = e & 63;
+      const bool in = c0 + col < N;
+      const z64 *g = F + (size_t)(k + nu * ND2) * N + c0 + col;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(Bs + buf * L::B_ELEMS + k * L::LDB + col)),
+                   "l"(in ? g : F), "r"(in ? 16 : 0));
+    }
+    asm volatile("cp.async.commit_group;");
+  };
+  // this thread's elements of sw: (row, i3) with i1 fastest, as chi0^q lies in memory
+  z64 pq[NE];
+  auto load_sw = [&](int nu) {
+#pragma unroll
+    for (int q = 0; q < NE; ++q) {
+      const int e = t + 128 * q, i3 = e / 32, m = m0 + e % 32;
+      if (e < 32 * ND2 && m < rows)
+        pq[q] = chi0q[((size_t)(m / ND2) * nnu + nu) * ND2 * ND2 + m % ND2 + i3 * ND2];
+    }
+  };
+  auto store_sw = [&](int nu, int buf) {
+#pragma unroll
+    for (int q = 0; q < NE; ++q) {
+      const int e = t + 128 * q, i3 = e / 32, r = e % 32, m = m0 + r;
+      if (e < 32 * ND2 && m < rows) {
+        z64 v = cmul(pq[q], c0inv[nu * ND2 + i3]);
+        if (m % ND2 == i3) v.x -= 1.0;
+        As[buf * L::A_ELEMS + r * L::LDA + i3] = v;
+        if (vterm) {
+          const z64 *cq = chi0q + ((size_t)(m / ND2) * nnu + nu) * ND2 * ND2 + m % ND2;
+          const z64 *vq = c.vq + (size_t)qidx[m / ND2] * ND2 * ND2 + i3 * ND2;
+          z64 s = czero<z64>();
+          for (int k = 0; k < ND2; ++k) cfma(s, cq[k * ND2], vq[k]);
+          Vs[buf * L::A_ELEMS + r * L::LDA + i3] = cscale(s, 2.0 / (c.beta * c.beta));
+        }
+      }
+    }
+  };
+  if (vterm)
+    for (int e = t; e < ND2 * 64; e += 128) {
+      const int k = e % ND2, col = e / ND2;
+      if (c0 + col < N) Og[k * L::LDB + col] = opg[k + (size_t)(c0 + col) * ND2];
+    }
+  // warp (wm, wn): rows 16 wm.., columns 32 wn..
+  const int wm = warp & 1, wn = warp >> 1, kl = lane & 3;
+  const int ra = 16 * wm + (lane >> 2), cb = 32 * wn + (lane >> 2);
+  double re[2][4][2], im[2][4][2], gr[GQ ? 2 : 1][4][2], gi[GQ ? 2 : 1][4][2];
+#pragma unroll
+  for (int i = 0; i < (GQ ? 2 : 1); ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) gr[i][j][0] = gr[i][j][1] = gi[i][j][0] = gi[i][j][1] = 0.0;
+  auto product = [&](const z64 *A, const z64 *B) {
+#pragma unroll
+    for (int k = 0; k < KP; k += 4) {
+      z64 a[2], b[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) a[i] = A[(ra + 8 * i) * L::LDA + k + kl];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = B[(k + kl) * L::LDB + cb + 8 * j];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const double an = -a[i].y;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          zg::dmma(re[i][j], a[i].x, b[j].x);
+          zg::dmma(im[i][j], a[i].x, b[j].y);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          zg::dmma(re[i][j], an, b[j].y);
+          zg::dmma(im[i][j], a[i].y, b[j].x);
+        }
+      }
+    }
+  };
+  stage_f(0, 0);
+  load_sw(0);
+  store_sw(0, 0);
+  for (int nu = 0; nu < nnu; ++nu) {
+    const int buf = nu & 1;
+    const bool more = nu + 1 < nnu;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                   // stage nu complete, stage nu - 1 read
+    if (more) {
+      stage_f(nu + 1, buf ^ 1);
+      load_sw(nu + 1);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
+    product(As + buf * L::A_ELEMS, Bs + buf * L::B_ELEMS);
+    if constexpr (GQ) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            gr[i][j][e] += re[i][j][e];
+            gi[i][j][e] += im[i][j][e];
+          }
+      if (vterm) product(Vs + buf * L::A_ELEMS, Og);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int m = m0 + ra + 8 * i, r = m % ND2 + nu * ND2;
+      if (m >= rows) continue;
+      TW *o = Tm + (size_t)(2 * (m / ND2) + ch) * strideM + (size_t)r * N;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int cc = c0 + 32 * wn + 8 * j + 2 * kl;       // even, N is even
+        if (cc >= N) continue;
+        const z64 t0 = make_double2((r == cc ? 1.0 : 0.0) - re[i][j][0], -im[i][j][0]);
+        const z64 t1 = make_double2((r == cc + 1 ? 1.0 : 0.0) - re[i][j][1], -im[i][j][1]);
+        if constexpr (sizeof(TW) == sizeof(z32))
+          *reinterpret_cast<float4 *>(o + cc) = make_float4((float)t0.x, (float)t0.y, (float)t1.x, (float)t1.y);
+        else {
+          o[cc] = t0;
+          o[cc + 1] = t1;
+        }
+      }
+    }
+    if (more) store_sw(nu + 1, buf ^ 1);
+  }
+  // the right-hand sides, and gamma^q_d
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int m = m0 + ra + 8 * i, p = m / ND2, i1 = m % ND2;
+    if (m >= rows) continue;
+    TW *o = Tm + (size_t)(2 * p + ch) * strideM + (size_t)(N + i1) * N;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int cc = c0 + 32 * wn + 8 * j + 2 * kl + e;
+        if (cc >= N) continue;
+        o[cc] = from64<TW>(opg[i1 + (size_t)cc * ND2]);
+        if constexpr (GQ)
+          if (gammaqd) gammaqd[(size_t)p * ND2 * N + i1 + (size_t)cc * ND2] = make_double2(gr[i][j][e], gi[i][j][e]);
+      }
+  }
+}
+
+// Two and three orbitals without the V(q) term: one block per (128-column tile, P points) of one
+// channel, on the CUDA cores: with K = nd2 = 4 or 9 the tensor-core form above spends a quarter of its
+// products on padding and waits at its per-nu barrier (density and magnetic channel of 250 points,
+// N = 1080, FP64: 1.48 and 1.38 ms here, 2.52 and 1.85 ms there).  A thread owns one column c of T; the F~ rows of each nu block are
 // staged into shared memory one nu ahead by cp.async (each thread copies and
 // reads only its own column), and sw_nu of the block's points is formed in
 // shared memory one nu ahead from chi0^q / chi0_loc^-1 values prefetched into
@@ -225,55 +377,63 @@ cudaError_t launch_to32(size_t n, const z64 *x, z32 *y, cudaStream_t st) {
   return ADGA_LAUNCH_CHECK();
 }
 
+template <typename T, int ND2, bool GQ>
+static cudaError_t launch_build_tile(const DevCtx &c, int npts, const z64 *chi0q, const z64 *c0inv, const z64 *F,
+                                     const z64 *opg, T *Tmat, size_t strideM, z64 *gammaqd, const int *qidx,
+                                     cudaStream_t st) {
+  typedef BuildTile<ND2> L;
+  cudaError_t e = smem_limit(k_bse_build<T, ND2, GQ>, L::smem(true));
+  if (e != cudaSuccess) return e;
+  const dim3 g(cdiv_u(c.N, 64), cdiv_u((size_t)npts * ND2, 32));
+  k_bse_build<T, ND2, GQ><<<g, 128, L::smem(GQ && c.vq), st>>>(c, npts, GQ ? 0 : 1, chi0q, c0inv, F, opg, Tmat,
+                                                             strideM, GQ ? gammaqd : nullptr, qidx);
+  return ADGA_LAUNCH_CHECK();
+}
+
 template <typename T>
 cudaError_t launch_bse_build(const DevCtx &c, int npts, const z64 *chi0q, const z64 *c0inv,
                              const z64 *Frow_d, const z64 *Frow_m, const z64 *opg_d,
                              const z64 *opg_m, T *Tmat, size_t strideM, z64 *gammaqd,
                              const int *qidx, cudaStream_t st, const z32 *F32_m) {
   if (npts <= 0) return cudaSuccess;
-  if (!c.vq && c.nd2 <= 9) {
-    cudaError_t e = cudaSuccess;
-#define FAST(NDD)                                                                                          \
-  {                                                                                                        \
-    dim3 g(cdiv_u(c.N, 128), cdiv_u(npts, BuildP<NDD, true>::P));                                         \
-    k_bse_build_fast<T, NDD, false, true><<<g, 128, 0, st>>>(c, npts, 0, chi0q, c0inv, Frow_d, opg_d,      \
-                                                             Tmat, strideM, gammaqd);                      \
-    if ((e = ADGA_LAUNCH_CHECK()) != cudaSuccess) return e;                                                \
-    g.y = cdiv_u(npts, BuildP<NDD, false>::P);                                                             \
-    bool done = false;                                                                                     \
-    if constexpr (std::is_same<T, z32>::value) {                                                           \
-      if (F32_m) {                                                                                         \
-        k_bse_build_fast<T, NDD, true, false><<<g, 128, 0, st>>>(c, npts, 1, chi0q, c0inv, F32_m, opg_m,   \
-                                                                 Tmat, strideM, nullptr);                  \
-        done = true;                                                                                       \
-      }                                                                                                    \
-    }                                                                                                      \
-    if (!done)                                                                                             \
-      k_bse_build_fast<T, NDD, false, false><<<g, 128, 0, st>>>(c, npts, 1, chi0q, c0inv, Frow_m, opg_m,   \
-                                                                Tmat, strideM, nullptr);                   \
+  if (c.nd2 == 1) {
+    k_bse_build_1<T><<<dim3(cdiv_u(c.N, 32), 2, npts), 256, 0, st>>>(c, chi0q, c0inv, Frow_d, Frow_m, opg_d, opg_m,
+                                                                    Tmat, strideM, gammaqd, qidx);
+    return ADGA_LAUNCH_CHECK();
   }
-    switch (c.nd2) {      // nd <= 3; larger orbital counts take the general kernel below
-      case 1: FAST(1); break;
-      case 4: FAST(4); break;
-      case 9: FAST(9); break;
-    }
-#undef FAST
-    if (c.nd2 <= 9) return ADGA_LAUNCH_CHECK();
-  }
-  dim3 grid(cdiv_u(c.N, 128), 2, npts);
-#define BUILD(NDD)                                                                            \
-  k_bse_build<T, NDD><<<grid, 128, 0, st>>>(c, chi0q, c0inv, Frow_d, Frow_m, opg_d, opg_m,     \
-                                            Tmat, strideM, gammaqd, qidx)
+  cudaError_t e = cudaErrorInvalidValue;
+#define TILE(NDD, GQ)                                                                                            \
+  launch_build_tile<T, NDD, GQ>(c, npts, chi0q, c0inv, GQ ? Frow_d : Frow_m, GQ ? opg_d : opg_m, Tmat, strideM,  \
+                                gammaqd, qidx, st)
+#define FAST(NDD, F32, GQ, F)                                                                                    \
+  (k_bse_build_fast<T, NDD, F32, GQ><<<dim3(cdiv_u(c.N, 128), cdiv_u(npts, BuildP<NDD, GQ>::P)), 128, 0, st>>>(  \
+       c, npts, GQ ? 0 : 1, chi0q, c0inv, F, GQ ? opg_d : opg_m, Tmat, strideM, GQ ? gammaqd : nullptr),         \
+   ADGA_LAUNCH_CHECK())
+#define BUILD_FAST(NDD)                                                                                          \
+  do {                                                                                                           \
+    e = c.vq ? TILE(NDD, true) : FAST(NDD, false, true, Frow_d);                                                 \
+    if (e != cudaSuccess) return e;                                                                              \
+    if constexpr (std::is_same<T, z32>::value) {                                                                 \
+      if (F32_m && !c.vq) return FAST(NDD, true, false, F32_m);                                                  \
+    }                                                                                                            \
+    e = FAST(NDD, false, false, Frow_m);                                                                         \
+  } while (0)
+#define BUILD_TILE(NDD)                                                                                          \
+  do {                                                                                                           \
+    e = TILE(NDD, true);                                                                                         \
+    if (e == cudaSuccess) e = TILE(NDD, false);                                                                  \
+  } while (0)
   switch (c.nd2) {
-    case 1: BUILD(1); break;
-    case 4: BUILD(4); break;
-    case 9: BUILD(9); break;
-    case 16: BUILD(16); break;
-    case 25: BUILD(25); break;
-    default: return cudaErrorInvalidValue;
+    case 4: BUILD_FAST(4); break;
+    case 9: BUILD_FAST(9); break;
+    case 16: BUILD_TILE(16); break;
+    case 25: BUILD_TILE(25); break;
   }
-#undef BUILD
-  return ADGA_LAUNCH_CHECK();
+#undef TILE
+#undef FAST
+#undef BUILD_FAST
+#undef BUILD_TILE
+  return e;
 }
 template cudaError_t launch_bse_build<z64>(const DevCtx &, int, const z64 *, const z64 *,
                                            const z64 *, const z64 *, const z64 *, const z64 *,
