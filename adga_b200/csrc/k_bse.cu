@@ -10,8 +10,11 @@
 //               (src/eom_module.f90:209-230), one owner thread per (k, nu).
 #include "ctx.cuh"
 #include "zgemm.cuh"
+#include <cooperative_groups.h>
 #include <algorithm>
 #include <type_traits>
+
+namespace cg = cooperative_groups;
 
 // ---------------------------------------------------------------------------
 // build: T(c, r) = delta(c, r) - sum_i3 sw_nu(i1, i3) F~(i3 + nu*nd2, c), r = i1 + nu*nd2,
@@ -443,100 +446,197 @@ template cudaError_t launch_bse_build<z32>(const DevCtx &, int, const z64 *, con
                                            z32 *, size_t, z64 *, const int *, cudaStream_t, const z32 *);
 
 // ---------------------------------------------------------------------------
-// post: one block per point.
+// post: one cluster of S blocks per point, the blocks sharing its frequencies.
 //   X_ch(c, i1) (column-major, ld ldX) = ((1+gamma^w) A^-1)^T  -> eta = X^T - (1+gamma^w)
 //   chi_ch = beta^-2 sum gamma (chi0q - chi0w) + beta^-2 sum eta chi0q
 //   m_tot(:, nu >= 0 half) = -(u - u~/2) eta_d/(beta nqp) + 1.5 u~ eta_m/(beta nqp)
 //                            + u gamma^q_d/(beta nqp)
+// A block stages VB frequencies at a time (chi0^q and both channels' eta, which it transposes for the
+// output on the way) and every product runs on ND x ND register tiles, so that an operand read from
+// shared memory feeds ND products: thread (g, ch, ib, jb) owns rows ib + ND r and columns jb + ND s of
+// frequency g of the stage.  The chi tiles stay in registers over all stages and are added over g and
+// then over the blocks in rank order.  Bound by the shared-memory reads and, for a few points, by the
+// stages' latency.
+// One block per point with eight lanes per chi element and a thread per m_tot element, operands from
+// global memory: 3.04 ms (216 points, 25 components, 40 frequencies), 1.78 ms (1000 points, 9, 120),
+// 0.30 ms (one of those); this kernel: 1.13 ms, 0.79 ms and 55 us.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
+template <int ND> struct PostTile {
+  static constexpr int ND2 = ND * ND, ND4 = ND2 * ND2;
+  static constexpr int VB = ND == 1 ? 64 : ND == 2 ? 16 : ND == 3 ? 7 : ND == 4 ? 4 : 2;   // frequencies per stage
+  static constexpr int ACT = 2 * ND2 * VB, NT = (ACT + 31) / 32 * 32;
+  static constexpr int LE = VB * ND2 + 1;                        // row stride of the staged eta
+  static constexpr size_t STAGE = (size_t)VB * ND4 + 2 * ND2 * LE;   // chi0^q, eta_d, eta_m
+  static constexpr size_t RED = (size_t)ACT * ND2;                // the threads' chi tiles
+  static constexpr int SMEM = (int)sizeof(z64) * (int)((STAGE > RED ? STAGE : RED) + 2 * ND4);
+};
+
+template <int ND>
+__global__ void __launch_bounds__(PostTile<ND>::NT)
 k_post(DevCtx c, const z64 *__restrict__ X, size_t sp, size_t sc, int ldX, const z64 *__restrict__ opg_d,
        const z64 *__restrict__ opg_m, const z64 *__restrict__ gam_d, const z64 *__restrict__ gam_m,
        const z64 *__restrict__ gammaqd, const z64 *__restrict__ chi0q, const z64 *__restrict__ c0w,
        z64 *chi_qw_d, z64 *chi_qw_m, z64 *mtot, z64 *etad, z64 *etam, const int *__restrict__ qidx) {
-  const int p = blockIdx.x;
-  const int N = c.N, nd2 = c.nd2, iwf = c.iwf;
-  const size_t nd2N = (size_t)nd2 * N;
-  z64 *ed = etad + p * nd2N, *em = etam + p * nd2N;
-  const z64 *Xd = X + (size_t)p * sp, *Xm = Xd + sc;
-  // 1. eta
-  for (size_t e = threadIdx.x; e < nd2N; e += blockDim.x) {
-    int i1 = (int)(e % nd2), cc = (int)(e / nd2);
-    ed[e] = csub(Xd[cc + (size_t)i1 * ldX], opg_d[e]);
-    em[e] = csub(Xm[cc + (size_t)i1 * ldX], opg_m[e]);
+  typedef PostTile<ND> L;
+  constexpr int ND2 = L::ND2, ND4 = L::ND4, VB = L::VB, NT = L::NT, LE = L::LE;
+  extern __shared__ __align__(16) z64 post_smem[];
+  z64 *uw = post_smem, *ut = uw + ND4;          // v + u - u~/2 and u~
+  z64 *Cs = ut + ND4, *Es = Cs + VB * ND4;      // [VB][i2][i3] and [ch][i1][LE]
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), S = (int)cl.num_blocks();
+  const int p = blockIdx.y, t = threadIdx.x, nnu = 2 * c.iwf, N = c.N;
+  const size_t nd2N = (size_t)ND2 * N;
+  const z64 *c0 = chi0q + (size_t)p * ND4 * nnu, *gq = gammaqd + (size_t)p * nd2N;
+  // V(q) terms of m_tot (src/eom_module.f90:187-205)
+  const z64 *vq = (mtot && c.vq && qidx) ? c.vq + (size_t)qidx[p] * ND4 : nullptr;
+  for (int e = t; e < ND4; e += NT) {
+    const z64 uu = c.u[e], tt = c.ut[e];
+    z64 w = make_double2(uu.x - 0.5 * tt.x, uu.y - 0.5 * tt.y);
+    if (vq) w = cadd(vq[e], w);                 // u_work = v + u - u~/2
+    uw[e] = w;
+    ut[e] = tt;
   }
-  __syncthreads();
-  const z64 *c0 = chi0q + (size_t)p * nd2 * nd2 * 2 * iwf;
-  const double b2 = c.beta * c.beta;
-  // 2. chi sums: eight lanes per (i1, i2, channel), lane l of the group summing the
-  //    frequencies dum = l mod 8, then a shuffle reduction (every lane of a warp
-  //    runs the same rounds)
-  {
-    const int l8 = threadIdx.x & 7, grp = threadIdx.x >> 3, ngrp = blockDim.x >> 3;
-    const int total = 2 * nd2 * nd2;
-    for (int base = 0; base < total; base += ngrp) {
-      const int t = base + grp;
-      z64 s1 = make_double2(0.0, 0.0), s2 = make_double2(0.0, 0.0);
-      int ch = 0, e = 0;
-      if (t < total) {
-        ch = t / (nd2 * nd2);
-        e = t % (nd2 * nd2);
-        const int i1 = e % nd2, i2 = e / nd2;
-        const z64 *g = ch ? gam_m : gam_d;
-        const z64 *et = ch ? em : ed;
-        for (int dum = l8; dum < 2 * iwf; dum += 8) {
-          const z64 *cq = c0 + (size_t)dum * nd2 * nd2 + (size_t)i2 * nd2;
-          for (int i3 = 0; i3 < nd2; ++i3) {
-            const size_t col = (size_t)(i3 + dum * nd2) * nd2;
-            const z64 q = cq[i3];
-            z64 nl = q;
-            if (i3 == i2) nl = csub(q, c0w[dum * nd2 + i2]);
-            cfma(s1, g[i1 + col], nl);
-            cfma(s2, et[i1 + col], q);
-          }
-        }
+  const bool act = t < L::ACT;
+  const int jb = t % ND, ib = t / ND % ND, ch = t / ND2 % 2, g = t / (2 * ND2);
+  z64 acc[ND][ND];
+#pragma unroll
+  for (int r = 0; r < ND; ++r)
+#pragma unroll
+    for (int s = 0; s < ND; ++s) acc[r][s] = czero<z64>();
+  const double inv = 1.0 / c.beta / (double)c.nqp;
+  for (int v0 = rank * VB; v0 < nnu; v0 += S * VB) {
+    const int nv = min(VB, nnu - v0), w = nv * ND2;
+    __syncthreads();                            // the last stage is read
+    for (int e = t; e < nv * ND4; e += NT) Cs[e] = c0[(size_t)v0 * ND4 + e];
+    for (int e = t; e < 2 * ND2 * w; e += NT) {
+      const int row = e / w, col = e % w;       // row = ch nd2 + i1
+      Es[row * LE + col] = X[(size_t)p * sp + (row / ND2) * sc + (size_t)(row % ND2) * ldX + v0 * ND2 + col];
+    }
+    __syncthreads();
+    // eta = X^T - (1 + gamma^w), written with i1 fastest
+    for (int e = t; e < 2 * ND2 * w; e += NT) {
+      const int ce = e / (ND2 * w), r = e % (ND2 * w), i1 = r % ND2, col = r / ND2;
+      const size_t o = (size_t)(v0 * ND2 + col) * ND2 + i1;
+      z64 &x = Es[(ce * ND2 + i1) * LE + col];
+      x = csub(x, (ce ? opg_m : opg_d)[o]);
+      ((ce ? etam : etad) + p * nd2N)[o] = x;
+    }
+    __syncthreads();
+    if (!act || g >= nv) continue;
+    const int nu = v0 + g;
+    const z64 *C = Cs + g * ND4, *E = Es + ch * ND2 * LE + g * ND2;
+    const z64 *G = (ch ? gam_m : gam_d) + (size_t)nu * ND2 * ND2;
+#pragma unroll 1
+    for (int i3 = 0; i3 < ND2; ++i3) {
+      z64 q[ND];
+#pragma unroll
+      for (int s = 0; s < ND; ++s) q[s] = C[(jb + ND * s) * ND2 + i3];
+#pragma unroll
+      for (int r = 0; r < ND; ++r) {
+        const z64 x = E[(ib + ND * r) * LE + i3];
+#pragma unroll
+        for (int s = 0; s < ND; ++s) cfma(acc[r][s], x, q[s]);
       }
 #pragma unroll
-      for (int o = 4; o > 0; o >>= 1) {
-        s1.x += __shfl_xor_sync(0xffffffffu, s1.x, o);
-        s1.y += __shfl_xor_sync(0xffffffffu, s1.y, o);
-        s2.x += __shfl_xor_sync(0xffffffffu, s2.x, o);
-        s2.y += __shfl_xor_sync(0xffffffffu, s2.y, o);
+      for (int s = 0; s < ND; ++s)
+        if (jb + ND * s == i3) q[s] = csub(q[s], c0w[nu * ND2 + i3]);
+#pragma unroll
+      for (int r = 0; r < ND; ++r) {
+        const z64 x = __ldg(G + ib + ND * r + i3 * ND2);
+#pragma unroll
+        for (int s = 0; s < ND; ++s) cfma(acc[r][s], x, q[s]);
       }
-      if (t < total && l8 == 0) {
-        z64 *out = (ch ? chi_qw_m : chi_qw_d) + (size_t)p * nd2 * nd2 + e;
-        z64 v = make_double2(s1.x / b2, s1.y / b2);
-        *out = cadd(v, make_double2(s2.x / b2, s2.y / b2));
+    }
+    // m_tot of a frequency nu >= 0: rows ib + ND r, columns jb + ND s, one half of the columns per ch thread
+    if (mtot && nu >= c.iwf) {
+      const z64 *Ed = Es + g * ND2, *Em = Ed + ND2 * LE;
+#pragma unroll 1
+      for (int s = ch; s < ND; s += 2) {
+        const int j = jb + ND * s;
+        z64 a1[ND], a2[ND], a3[ND];
+#pragma unroll
+        for (int r = 0; r < ND; ++r) a1[r] = a2[r] = a3[r] = czero<z64>();
+#pragma unroll 1
+        for (int i3 = 0; i3 < ND2; ++i3) {
+          const z64 ed = Ed[i3 * LE + j], em = Em[i3 * LE + j], gv = __ldg(gq + i3 + (size_t)(nu * ND2 + j) * ND2);
+#pragma unroll
+          for (int r = 0; r < ND; ++r) {
+            const int i1 = ib + ND * r;
+            const z64 tt = ut[i1 + i3 * ND2];
+            cfma(a1[r], uw[i1 + i3 * ND2], ed);
+            cfma(a2[r], tt, em);
+            cfma(a3[r], __ldg(c.u + i1 + i3 * ND2), gv);
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < ND; ++r) {
+          const int i1 = ib + ND * r;
+          z64 v = cscale(a1[r], -inv);
+          v = cadd(cscale(a2[r], 1.5 * inv), v);
+          v = cadd(cscale(a3[r], inv), v);
+          if (vq) {                             // v gamma^w_d
+            z64 a4 = czero<z64>();
+            for (int i3 = 0; i3 < ND2; ++i3) cfma(a4, vq[i1 + i3 * ND2], gam_d[i3 + (size_t)(nu * ND2 + j) * ND2]);
+            v = cadd(cscale(a4, -inv), v);
+          }
+          mtot[(size_t)p * ND4 * c.iwf + i1 + (size_t)((nu - c.iwf) * ND2 + j) * ND2] = v;
+        }
       }
     }
   }
-  // 3. m_tot for the nu >= 0 half of the columns
-  if (mtot) {
-    const double inv = 1.0 / c.beta / (double)c.nqp;
-    // V(q) terms of m_tot (src/eom_module.f90:187-205)
-    const z64 *vq = (c.vq && qidx) ? c.vq + (size_t)qidx[p] * nd2 * nd2 : nullptr;
-    const z64 *gq = gammaqd + (size_t)p * nd2N;
-    z64 *m = mtot + (size_t)p * nd2 * iwf * nd2;
-    for (int t = threadIdx.x; t < nd2 * iwf * nd2; t += blockDim.x) {
-      int i1 = t % nd2, cl = t / nd2;          // local column
-      size_t col = (size_t)(cl + iwf * nd2) * nd2;
-      z64 a1 = make_double2(0.0, 0.0), a2 = a1, a3 = a1, a4 = a1;
-      for (int i3 = 0; i3 < nd2; ++i3) {
-        z64 uu = c.u[i1 + i3 * nd2], tt = c.ut[i1 + i3 * nd2];
-        z64 uw = make_double2(uu.x - 0.5 * tt.x, uu.y - 0.5 * tt.y);
-        if (vq) uw = cadd(vq[i1 + i3 * nd2], uw);       // u_work = v + u - u~/2
-        cfma(a1, uw, ed[i3 + col]);
-        cfma(a2, tt, em[i3 + col]);
-        cfma(a3, uu, gq[i3 + col]);
-        if (vq) cfma(a4, vq[i1 + i3 * nd2], gam_d[i3 + col]);   // v gamma^w_d
-      }
-      z64 v = cscale(a1, -inv);
-      v = cadd(cscale(a2, 1.5 * inv), v);
-      v = cadd(cscale(a3, inv), v);
-      if (vq) v = cadd(cscale(a4, -inv), v);
-      m[t] = v;
+  // the tiles of all frequencies: over the stage's slots, then over the cluster's blocks
+  __syncthreads();
+  z64 *red = Cs;                                // [element][thread]
+  if (act)
+#pragma unroll
+    for (int r = 0; r < ND; ++r)
+#pragma unroll
+      for (int s = 0; s < ND; ++s) red[(r * ND + s) * L::ACT + t] = acc[r][s];
+  __syncthreads();
+  constexpr int OUT = 2 * ND4;
+  for (int e = t; e < OUT; e += NT) {
+    const int rs = e / (2 * ND2), th = e % (2 * ND2);
+    z64 v = czero<z64>();
+    for (int k = 0; k < VB; ++k) v = cadd(v, red[rs * L::ACT + k * 2 * ND2 + th]);
+    red[rs * L::ACT + th] = v;                  // slot 0 of the same (element, thread) column
+  }
+  cl.sync();
+  if (rank == 0) {
+    const double b2 = c.beta * c.beta;
+    for (int e = t; e < OUT; e += NT) {
+      const int rs = e / (2 * ND2), th = e % (2 * ND2);
+      z64 v = czero<z64>();
+      for (int k = 0; k < S; ++k) v = cadd(v, cl.map_shared_rank(red, k)[rs * L::ACT + th]);
+      const int i1 = th / ND % ND + ND * (rs / ND), i2 = th % ND + ND * (rs % ND);
+      (th / ND2 ? chi_qw_m : chi_qw_d)[(size_t)p * ND4 + i1 + i2 * ND2] = make_double2(v.x / b2, v.y / b2);
     }
   }
+  cl.sync();                                    // the first block has read the others' sums
+}
+
+template <int ND, typename... A>
+static cudaError_t launch_post_nd(int npts, int nnu, cudaStream_t st, A... args) {
+  typedef PostTile<ND> L;
+  cudaError_t e = smem_limit(k_post<ND>, L::SMEM);
+  if (e != cudaSuccess) return e;
+  // blocks for about two waves of two per SM, at least one stage each
+  const int stages = (nnu + L::VB - 1) / L::VB;
+  int S = 1;
+  while (S < 8 && 2 * S <= stages && 2 * S * npts <= 1184) S *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(S, npts);
+  cfg.blockDim = dim3(L::NT);
+  cfg.dynamicSmemBytes = L::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = S;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, k_post<ND>, args...);
+  if (e != cudaSuccess) return e;
+  return ADGA_LAUNCH_CHECK();
 }
 
 cudaError_t launch_post(const DevCtx &c, int npts, const z64 *X, size_t sp, size_t sc, int ldX,
@@ -544,9 +644,18 @@ cudaError_t launch_post(const DevCtx &c, int npts, const z64 *X, size_t sp, size
                         const z64 *gammaqd, const z64 *chi0q, const z64 *c0w, z64 *chi_qw_d,
                         z64 *chi_qw_m, z64 *mtot, z64 *etad, z64 *etam, const int *qidx, cudaStream_t st) {
   if (npts <= 0) return cudaSuccess;
-  k_post<<<npts, 256, 0, st>>>(c, X, sp, sc, ldX, opg_d, opg_m, gam_d, gam_m, gammaqd, chi0q, c0w,
-                               chi_qw_d, chi_qw_m, mtot, etad, etam, qidx);
-  return ADGA_LAUNCH_CHECK();
+#define POST(NDD)                                                                                                  \
+  return launch_post_nd<NDD>(npts, 2 * c.iwf, st, c, X, sp, sc, ldX, opg_d, opg_m, gam_d, gam_m, gammaqd, chi0q,   \
+                             c0w, chi_qw_d, chi_qw_m, mtot, etad, etam, qidx)
+  switch (c.nd) {
+    case 1: POST(1);
+    case 2: POST(2);
+    case 3: POST(3);
+    case 4: POST(4);
+    case 5: POST(5);
+  }
+#undef POST
+  return cudaErrorInvalidValue;
 }
 
 // ---------------------------------------------------------------------------

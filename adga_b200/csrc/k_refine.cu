@@ -28,27 +28,65 @@ __global__ void k_init_x(const z32 *T32, size_t strideM, int N, int R, int nmat,
   X[idx] = to64(T32[m * strideM + (size_t)N * N + e]);
 }
 
-// XD(i1, i3 + nu*nd2) = sum_i2 X(i1, i2 + nu*nd2) sw_nu(i2, i3), row-major R x N
-__global__ void k_xd(DevCtx c, int npts, const z64 *X, const z64 *chi0q, const z64 *c0inv, z64 *XD,
-                     int minus_one) {
-  const int nd2 = c.nd2, N = c.N;
-  size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  size_t per = (size_t)nd2 * N;
-  if (idx >= per * 2 * npts) return;
-  size_t m = idx / per, e = idx % per;
-  int i1 = (int)(e / N), col = (int)(e % N);
-  int nu = col / nd2, i3 = col % nd2;
-  int p = (int)(m >> 1);
-  const z64 *x = X + m * per + (size_t)i1 * N + (size_t)nu * nd2;
-  const z64 *cq = chi0q + (size_t)p * nd2 * nd2 * 2 * c.iwf + (size_t)nu * nd2 * nd2 + (size_t)i3 * nd2;
-  const z64 ci = c0inv[nu * nd2 + i3];
-  z64 s = make_double2(0.0, 0.0);
-  for (int i2 = 0; i2 < nd2; ++i2) {
-    z64 sw = cmul(cq[i2], ci);
-    if (i2 == i3 && minus_one) sw.x -= 1.0;
-    cfma(s, x[i2], sw);
+// XD(i1, i3 + nu*nd2) = sum_i2 X(i1, i2 + nu*nd2) sw_nu(i2, i3), row-major R x N.
+// A block takes VB frequencies of one point: sw (formed once for both channels) and the X rows are staged
+// in shared memory, thread (g, ch, ib, jb) owns the ND x ND outputs of rows ib + ND r and columns
+// jb + ND s of frequency g.  Bound by memory (X read, XD written); a thread per output with operands
+// and sw from global memory took 734 us a call (216 points, 25 components, 40 frequencies) and 528 us
+// (1000 points, 9, 120); this kernel: 173 us and 218 us.
+template <int ND> struct XdTile {
+  static constexpr int ND2 = ND * ND, ND4 = ND2 * ND2;
+  static constexpr int VB = ND == 1 ? 64 : ND == 2 ? 16 : ND == 3 ? 7 : ND == 4 ? 4 : 2;
+  static constexpr int ACT = 2 * ND2 * VB, NT = (ACT + 31) / 32 * 32, LX = VB * ND2 + 1;
+  static constexpr int SMEM = (int)sizeof(z64) * (VB * ND4 + 2 * ND2 * LX);
+};
+template <int ND>
+__global__ void __launch_bounds__(XdTile<ND>::NT)
+k_xd(DevCtx c, const z64 *__restrict__ X, const z64 *__restrict__ chi0q, const z64 *__restrict__ c0inv,
+     z64 *__restrict__ XD, int minus_one) {
+  typedef XdTile<ND> L;
+  constexpr int ND2 = L::ND2, ND4 = L::ND4, NT = L::NT, LX = L::LX;
+  extern __shared__ __align__(16) z64 xd_smem[];
+  z64 *Ss = xd_smem, *Xs = Ss + L::VB * ND4;        // [VB][i3][i2] and [ch][i1][LX]
+  const int t = threadIdx.x, N = c.N, nnu = 2 * c.iwf, p = blockIdx.y;
+  const int v0 = blockIdx.x * L::VB, nv = min(L::VB, nnu - v0), w = nv * ND2;
+  const size_t per = (size_t)ND2 * N, base = (size_t)2 * p * per + (size_t)v0 * ND2;
+  for (int e = t; e < nv * ND4; e += NT) {
+    const int i2 = e % ND2, r = e / ND2;             // r = g nd2 + i3
+    z64 s = cmul(chi0q[((size_t)p * nnu + v0) * ND4 + e], c0inv[v0 * ND2 + r]);
+    if (i2 == r % ND2 && minus_one) s.x -= 1.0;
+    Ss[e] = s;
   }
-  XD[m * per + e] = s;
+  for (int e = t; e < 2 * ND2 * w; e += NT) {
+    const int row = e / w, col = e % w;
+    Xs[row * LX + col] = X[base + (size_t)row * N + col];
+  }
+  __syncthreads();
+  const int jb = t % ND, ib = t / ND % ND, ch = t / ND2 % 2, g = t / (2 * ND2);
+  if (t >= L::ACT || g >= nv) return;
+  const z64 *sx = Xs + ch * ND2 * LX + g * ND2, *ss = Ss + g * ND4;
+  z64 acc[ND][ND];
+#pragma unroll
+  for (int r = 0; r < ND; ++r)
+#pragma unroll
+    for (int s = 0; s < ND; ++s) acc[r][s] = czero<z64>();
+#pragma unroll 1
+  for (int i2 = 0; i2 < ND2; ++i2) {
+    z64 y[ND];
+#pragma unroll
+    for (int s = 0; s < ND; ++s) y[s] = ss[(jb + ND * s) * ND2 + i2];
+#pragma unroll
+    for (int r = 0; r < ND; ++r) {
+      const z64 x = sx[(ib + ND * r) * LX + i2];
+#pragma unroll
+      for (int s = 0; s < ND; ++s) cfma(acc[r][s], x, y[s]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < ND; ++r)
+#pragma unroll
+    for (int s = 0; s < ND; ++s)
+      XD[base + (size_t)(ch * ND2 + ib + ND * r) * N + g * ND2 + jb + ND * s] = acc[r][s];
 }
 
 // X += up(V); per-matrix max |d| and max |X| (|re|+|im|) into norms[2*m], norms[2*m+1]
@@ -90,9 +128,7 @@ cudaError_t launch_residual(const DevCtx &c, int npts, const z64 *X, const z64 *
                             const z64 *opg_d, const z64 *opg_m, z64 *XD, z32 *V, const z64 *extra_d,
                             unsigned long long *rnorm, cudaStream_t st, const z64 *Bpt, void *ri8,
                             long long fgen) {
-  size_t total = (size_t)c.nd2 * c.N * 2 * npts;
-  k_xd<<<cdiv_u(total, 256), 256, 0, st>>>(c, npts, X, chi0q, c0inv, XD, 1);
-  cudaError_t e = ADGA_LAUNCH_CHECK();
+  cudaError_t e = launch_xd(c, npts, X, chi0q, c0inv, XD, true, st);
   if (e != cudaSuccess) return e;
   if (ri8)
     return ri8_residual(ri8, c, npts, XD, X, Frow_d, Frow_m, fgen, opg_d, opg_m, V, extra_d, rnorm, Bpt, st);
@@ -102,9 +138,24 @@ cudaError_t launch_residual(const DevCtx &c, int npts, const z64 *X, const z64 *
 // XD = X blockdiag(chi0q chi0_loc^-1 - 1), or without the -1 (a tangent direction)
 cudaError_t launch_xd(const DevCtx &c, int npts, const z64 *X, const z64 *chi0q, const z64 *c0inv, z64 *XD,
                       bool minus_one, cudaStream_t st) {
-  size_t total = (size_t)c.nd2 * c.N * 2 * npts;
-  k_xd<<<cdiv_u(total, 256), 256, 0, st>>>(c, npts, X, chi0q, c0inv, XD, minus_one ? 1 : 0);
-  return ADGA_LAUNCH_CHECK();
+  if (npts <= 0) return cudaSuccess;
+#define XDL(ND)                                                                                                   \
+  do {                                                                                                            \
+    typedef XdTile<ND> L;                                                                                         \
+    cudaError_t e = smem_limit(k_xd<ND>, L::SMEM);                                                                \
+    if (e != cudaSuccess) return e;                                                                               \
+    k_xd<ND><<<dim3(cdiv_u(2 * c.iwf, L::VB), npts), L::NT, L::SMEM, st>>>(c, X, chi0q, c0inv, XD, minus_one);    \
+    return ADGA_LAUNCH_CHECK();                                                                                   \
+  } while (0)
+  switch (c.nd) {
+    case 1: XDL(1);
+    case 2: XDL(2);
+    case 3: XDL(3);
+    case 4: XDL(4);
+    case 5: XDL(5);
+  }
+#undef XDL
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_update(int per, int nmat, const z32 *V, z64 *X, unsigned long long *norms,
