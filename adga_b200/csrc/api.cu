@@ -1217,7 +1217,7 @@ static int run_batch(adga_handle *h, int iwb, int np, int off, int prec, int *st
   if (prec == ADGA_FP64) {
     z64 *T = (z64 *)h->Tm;
     CK(launch_bse_build<z64>(c, np, chi0q, h->c0inv, h->Frow_d, h->Frow_m, h->opg_d, h->opg_m, T,
-                             strideM, h->gq, h->qidx_d, st));
+                             strideM, h->gq, h->qidx_d, h->etad, st));
     cudaEventRecord(ev[2], st);
     if (!h->tan_on && lu_small_supported((int)N, (int)R)) {
       CK(lu_small_solve(T, strideM, (int)N, (int)R, 2 * np, h->info, st));
@@ -1234,7 +1234,7 @@ static int run_batch(adga_handle *h, int iwb, int np, int off, int prec, int *st
       h->f32_iwb = iwb;
     }
     CK(launch_bse_build<z32>(c, np, chi0q, h->c0inv, h->Frow_d, h->Frow_m, h->opg_d, h->opg_m, T,
-                             strideM, h->gq, h->qidx_d, st, h->Frow32_m));
+                             strideM, h->gq, h->qidx_d, h->etad, st, h->Frow32_m));
     cudaEventRecord(ev[2], st);
     CK(factor_batch<z32>(h, T, lb, true, h->tc != nullptr, &tt, h->mixed_nopiv));
     // the solves of the FP32 factors on the tensor cores (tune.trsv_tc = 0: streaming solves)

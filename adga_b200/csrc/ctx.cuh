@@ -116,11 +116,12 @@ cudaError_t launch_chi0_finish(const DevCtx &c, const z64 *chi0_all, int nnu_all
                                const z64 *bubloc_tmp, z64 *chi0q, z64 *bubble_nl, cudaStream_t st);
 
 // k_bse.cu
+// vscr: room for npts x 2 iwf x nd2 x nd2 elements (used with V(q))
 template <typename T>
 cudaError_t launch_bse_build(const DevCtx &c, int npts, const z64 *chi0q, const z64 *c0inv,
                              const z64 *Frow_d, const z64 *Frow_m, const z64 *opg_d,
                              const z64 *opg_m, T *Tmat, size_t strideM, z64 *gammaqd,
-                             const int *qidx, cudaStream_t st, const z32 *F32_m = nullptr);
+                             const int *qidx, z64 *vscr, cudaStream_t st, const z32 *F32_m = nullptr);
 // FP32 copy of an N x N FP64 matrix (the magnetic F~ of the mixed build)
 cudaError_t launch_to32(size_t n, const z64 *x, z32 *y, cudaStream_t st);
 // X of point p, channel ch at X + p*sp + ch*sc: N x R column-major (ld ldX)

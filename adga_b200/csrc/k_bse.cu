@@ -61,6 +61,19 @@ k_bse_build_1(DevCtx c, const z64 *__restrict__ chi0q, const z64 *__restrict__ c
   }
 }
 
+// 2 beta^-2 chi0^q(nu) v(q) for every point and frequency, in chi0^q's layout (src/main.F90:710-719)
+__global__ void k_vq_sv(DevCtx c, size_t n, const z64 *__restrict__ chi0q, const int *__restrict__ qidx,
+                        z64 *__restrict__ sv) {
+  const size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (idx >= n) return;
+  const int nd2 = c.nd2, nd4 = nd2 * nd2, i1 = (int)(idx % nd2), i3 = (int)(idx / nd2 % nd2);
+  const z64 *cq = chi0q + idx / nd4 * nd4 + i1;
+  const z64 *vq = c.vq + (size_t)qidx[idx / nd4 / (2 * c.iwf)] * nd4 + (size_t)i3 * nd2;
+  z64 s = czero<z64>();
+  for (int k = 0; k < nd2; ++k) cfma(s, cq[k * nd2], vq[k]);
+  sv[idx] = cscale(s, 2.0 / (c.beta * c.beta));
+}
+
 // Four and five orbitals, and the density channel with V(q): per nu a product of the batch's sw rows (npts nd2 x nd2) with the nd2 x N block of F~
 // on the FP64 tensor cores (m8n8k4, complex as four real products).  A CTA owns 32 rows (p, i1) and 64
 // columns and walks nu: F~'s block of the next nu arrives by cp.async while sw of the next nu is formed
@@ -71,7 +84,7 @@ k_bse_build_1(DevCtx c, const z64 *__restrict__ chi0q, const z64 *__restrict__ c
 // operand, after gamma^q_d has taken the first.
 // A thread per column with all products on the CUDA cores took 8.8 ms (both channels, 216 points,
 // N = 1000, 25 components; this kernel 4.45 ms) and 0.81 ms (both, 216 points, N = 486, with V(q); this
-// kernel for the density channel 0.62 ms, the magnetic one as without V(q) 0.25 ms).
+// kernel for the density channel 0.51 ms, the magnetic one as without V(q) 0.25 ms).
 template <int ND2> struct BuildTile {
   static constexpr int KP = (ND2 + 3) / 4 * 4;
   static constexpr int LDA = KP % 8 == 4 ? KP : KP + 4, LDB = 66;      // conflict-free fragment reads
@@ -85,7 +98,7 @@ template <typename TW, int ND2, bool GQ>
 __global__ void __launch_bounds__(128, 2)
 k_bse_build(DevCtx c, int npts, int ch, const z64 *__restrict__ chi0q, const z64 *__restrict__ c0inv,
             const z64 *__restrict__ F, const z64 *__restrict__ opg, TW *Tm, size_t strideM, z64 *gammaqd,
-            const int *__restrict__ qidx) {
+            const z64 *__restrict__ sv) {
   typedef BuildTile<ND2> L;
   constexpr int KP = L::KP, NE = (32 * ND2 + 127) / 128;
   extern __shared__ __align__(16) z64 bse_smem[];
@@ -107,13 +120,16 @@ k_bse_build(DevCtx c, int npts, int ch, const z64 *__restrict__ chi0q, const z64
     asm volatile("cp.async.commit_group;");
   };
   // this thread's elements of sw: (row, i3) with i1 fastest, as chi0^q lies in memory
-  z64 pq[NE];
+  z64 pq[NE], pv[NE];
   auto load_sw = [&](int nu) {
 #pragma unroll
     for (int q = 0; q < NE; ++q) {
       const int e = t + 128 * q, i3 = e / 32, m = m0 + e % 32;
-      if (e < 32 * ND2 && m < rows)
-        pq[q] = chi0q[((size_t)(m / ND2) * nnu + nu) * ND2 * ND2 + m % ND2 + i3 * ND2];
+      if (e < 32 * ND2 && m < rows) {
+        const size_t at = ((size_t)(m / ND2) * nnu + nu) * ND2 * ND2 + m % ND2 + i3 * ND2;
+        pq[q] = chi0q[at];
+        if (vterm) pv[q] = sv[at];
+      }
     }
   };
   auto store_sw = [&](int nu, int buf) {
@@ -124,13 +140,7 @@ k_bse_build(DevCtx c, int npts, int ch, const z64 *__restrict__ chi0q, const z64
         z64 v = cmul(pq[q], c0inv[nu * ND2 + i3]);
         if (m % ND2 == i3) v.x -= 1.0;
         As[buf * L::A_ELEMS + r * L::LDA + i3] = v;
-        if (vterm) {
-          const z64 *cq = chi0q + ((size_t)(m / ND2) * nnu + nu) * ND2 * ND2 + m % ND2;
-          const z64 *vq = c.vq + (size_t)qidx[m / ND2] * ND2 * ND2 + i3 * ND2;
-          z64 s = czero<z64>();
-          for (int k = 0; k < ND2; ++k) cfma(s, cq[k * ND2], vq[k]);
-          Vs[buf * L::A_ELEMS + r * L::LDA + i3] = cscale(s, 2.0 / (c.beta * c.beta));
-        }
+        if (vterm) Vs[buf * L::A_ELEMS + r * L::LDA + i3] = pv[q];
       }
     }
   };
@@ -382,14 +392,14 @@ cudaError_t launch_to32(size_t n, const z64 *x, z32 *y, cudaStream_t st) {
 
 template <typename T, int ND2, bool GQ>
 static cudaError_t launch_build_tile(const DevCtx &c, int npts, const z64 *chi0q, const z64 *c0inv, const z64 *F,
-                                     const z64 *opg, T *Tmat, size_t strideM, z64 *gammaqd, const int *qidx,
+                                     const z64 *opg, T *Tmat, size_t strideM, z64 *gammaqd, const z64 *sv,
                                      cudaStream_t st) {
   typedef BuildTile<ND2> L;
   cudaError_t e = smem_limit(k_bse_build<T, ND2, GQ>, L::smem(true));
   if (e != cudaSuccess) return e;
   const dim3 g(cdiv_u(c.N, 64), cdiv_u((size_t)npts * ND2, 32));
   k_bse_build<T, ND2, GQ><<<g, 128, L::smem(GQ && c.vq), st>>>(c, npts, GQ ? 0 : 1, chi0q, c0inv, F, opg, Tmat,
-                                                             strideM, GQ ? gammaqd : nullptr, qidx);
+                                                             strideM, GQ ? gammaqd : nullptr, sv);
   return ADGA_LAUNCH_CHECK();
 }
 
@@ -397,7 +407,7 @@ template <typename T>
 cudaError_t launch_bse_build(const DevCtx &c, int npts, const z64 *chi0q, const z64 *c0inv,
                              const z64 *Frow_d, const z64 *Frow_m, const z64 *opg_d,
                              const z64 *opg_m, T *Tmat, size_t strideM, z64 *gammaqd,
-                             const int *qidx, cudaStream_t st, const z32 *F32_m) {
+                             const int *qidx, z64 *vscr, cudaStream_t st, const z32 *F32_m) {
   if (npts <= 0) return cudaSuccess;
   if (c.nd2 == 1) {
     k_bse_build_1<T><<<dim3(cdiv_u(c.N, 32), 2, npts), 256, 0, st>>>(c, chi0q, c0inv, Frow_d, Frow_m, opg_d, opg_m,
@@ -405,9 +415,14 @@ cudaError_t launch_bse_build(const DevCtx &c, int npts, const z64 *chi0q, const 
     return ADGA_LAUNCH_CHECK();
   }
   cudaError_t e = cudaErrorInvalidValue;
+  if (c.vq) {
+    const size_t n = (size_t)npts * 2 * c.iwf * c.nd2 * c.nd2;
+    k_vq_sv<<<cdiv_u(n, 256), 256, 0, st>>>(c, n, chi0q, qidx, vscr);
+    if ((e = ADGA_LAUNCH_CHECK()) != cudaSuccess) return e;
+  }
 #define TILE(NDD, GQ)                                                                                            \
   launch_build_tile<T, NDD, GQ>(c, npts, chi0q, c0inv, GQ ? Frow_d : Frow_m, GQ ? opg_d : opg_m, Tmat, strideM,  \
-                                gammaqd, qidx, st)
+                                gammaqd, vscr, st)
 #define FAST(NDD, F32, GQ, F)                                                                                    \
   (k_bse_build_fast<T, NDD, F32, GQ><<<dim3(cdiv_u(c.N, 128), cdiv_u(npts, BuildP<NDD, GQ>::P)), 128, 0, st>>>(  \
        c, npts, GQ ? 0 : 1, chi0q, c0inv, F, GQ ? opg_d : opg_m, Tmat, strideM, GQ ? gammaqd : nullptr),         \
@@ -440,10 +455,12 @@ cudaError_t launch_bse_build(const DevCtx &c, int npts, const z64 *chi0q, const 
 }
 template cudaError_t launch_bse_build<z64>(const DevCtx &, int, const z64 *, const z64 *,
                                            const z64 *, const z64 *, const z64 *, const z64 *,
-                                           z64 *, size_t, z64 *, const int *, cudaStream_t, const z32 *);
+                                           z64 *, size_t, z64 *, const int *, z64 *, cudaStream_t,
+                                           const z32 *);
 template cudaError_t launch_bse_build<z32>(const DevCtx &, int, const z64 *, const z64 *,
                                            const z64 *, const z64 *, const z64 *, const z64 *,
-                                           z32 *, size_t, z64 *, const int *, cudaStream_t, const z32 *);
+                                           z32 *, size_t, z64 *, const int *, z64 *, cudaStream_t,
+                                           const z32 *);
 
 // ---------------------------------------------------------------------------
 // post: one cluster of S blocks per point, the blocks sharing its frequencies.
