@@ -14,6 +14,8 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -112,6 +114,13 @@ struct adga_handle {
   adga_tune tune{0, 2, 1, 0, 1, 1};   // mixed-path kernel choices (adga_set_tune / adga_autotune)
   void *ri8 = nullptr;            // int8-slice residual context (k_resid_i8.cu), with the mixed work
   long long frow_gen = 0;         // bumped whenever F~ is recomputed (its residual slices go stale)
+  // work buffer of the single-call entry points (grown on demand), the events of a batch, and the
+  // page-locked buffer of large downloads
+  char *scr = nullptr;
+  size_t scr_cap = 0;
+  std::vector<cudaEvent_t> events;
+  char *stage = nullptr;
+  cudaEvent_t stage_ev[2 * 4] = {};
   // last-run statistics
   adga_run_stats stats{};
 };
@@ -175,6 +184,110 @@ static bool alloc_into(adga_handle *h, P *&ptr, size_t count, std::vector<void *
 static void free_list(std::vector<void *> &list) {
   for (void *p : list) cudaFree(p);
   list.clear();
+}
+
+// room for `bytes` in the handle's work buffer, valid until the next call that asks for more
+static char *scratch(adga_handle *h, size_t bytes) {
+  if (h->scr_cap < bytes) {
+    cudaStreamSynchronize(h->st);
+    if (h->scr) cudaFree(h->scr);
+    h->scr = nullptr;
+    h->scr_cap = 0;
+    if (cudaMalloc(&h->scr, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      h->scr = nullptr;
+      return nullptr;
+    }
+    h->scr_cap = bytes;
+  }
+  return h->scr;
+}
+// the parts of one scratch buffer, 16-byte elements
+static bool scratch_parts(adga_handle *h, std::initializer_list<std::pair<z64 **, size_t>> parts) {
+  size_t n = 0;
+  for (auto &x : parts) n += x.second;
+  z64 *p = (z64 *)scratch(h, std::max<size_t>(n, 1) * sizeof(z64));
+  if (!p) return false;
+  for (auto &x : parts) {
+    *x.first = p;
+    p += x.second;
+  }
+  return true;
+}
+
+// the first n events of the handle's pool (a batch's timing)
+static cudaEvent_t *batch_events(adga_handle *h, size_t n) {
+  while (h->events.size() < n) {
+    cudaEvent_t e = nullptr;
+    if (cudaEventCreate(&e) != cudaSuccess) return nullptr;
+    h->events.push_back(e);
+  }
+  return h->events.data();
+}
+
+// Device to host on the handle's stream.  A large copy into pageable memory would run through the
+// driver's own staging on one thread, which also takes the page faults of a fresh array (21 MB: 5.2 ms);
+// four threads with two page-locked chunks each copy and fault in parallel (2.6 ms).  Complete on return
+// in that case; smaller or page-locked copies stay asynchronous.
+constexpr int kStageThreads = 4;
+constexpr size_t kStageChunk = 512 * 1024, kStageMin = 4 * 1024 * 1024;
+static cudaError_t download(adga_handle *h, void *dst, const void *src, size_t bytes) {
+  cudaPointerAttributes at{};
+  if (bytes < kStageMin || cudaPointerGetAttributes(&at, dst) != cudaSuccess ||
+      at.type != cudaMemoryTypeUnregistered) {
+    cudaGetLastError();
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->st);
+  }
+  if (!h->stage) {
+    if (cudaMallocHost(&h->stage, 2 * kStageThreads * kStageChunk) != cudaSuccess) {
+      cudaGetLastError();
+      h->stage = nullptr;
+      return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->st);
+    }
+  }
+  for (cudaEvent_t &e : h->stage_ev)
+    if (!e) {
+      cudaError_t r = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+      if (r != cudaSuccess) return r;
+    }
+  int dev = 0;
+  cudaError_t r = cudaGetDevice(&dev);
+  if (r != cudaSuccess) return r;
+  cudaError_t res[kStageThreads] = {};
+  const size_t nch = (bytes + kStageChunk - 1) / kStageChunk;
+  // thread w copies the chunks w, w + 4, ..: the next one is on its way while one is stored
+  auto work = [&](int w) {
+    cudaError_t e = cudaSetDevice(dev);
+    auto len = [&](size_t i) { return std::min(kStageChunk, bytes - i * kStageChunk); };
+    auto start = [&](size_t i, int b) {
+      e = cudaMemcpyAsync(h->stage + (2 * w + b) * kStageChunk, (const char *)src + i * kStageChunk, len(i),
+                          cudaMemcpyDeviceToHost, h->st);
+      if (e == cudaSuccess) e = cudaEventRecord(h->stage_ev[2 * w + b], h->st);
+    };
+    int b = 0;
+    if (e == cudaSuccess && (size_t)w < nch) start(w, 0);
+    for (size_t i = w; e == cudaSuccess && i < nch; i += kStageThreads, b ^= 1) {
+      if (i + kStageThreads < nch) start(i + kStageThreads, b ^ 1);
+      if (e == cudaSuccess) e = cudaEventSynchronize(h->stage_ev[2 * w + b]);
+      if (e == cudaSuccess) memcpy((char *)dst + i * kStageChunk, h->stage + (2 * w + b) * kStageChunk, len(i));
+    }
+    res[w] = e;
+  };
+  std::thread th[kStageThreads];
+  int started = 1;                                   // the caller's own share is 0
+  try {
+    for (; started < kStageThreads; ++started) th[started] = std::thread(work, started);
+  } catch (const std::system_error &) {
+  }
+  work(0);
+  for (int w = started; w < kStageThreads; ++w) work(w);     // threads that could not be started
+  for (int w = 1; w < started; ++w) th[w].join();
+  for (cudaError_t e : res)
+    if (e != cudaSuccess) {
+      cudaStreamSynchronize(h->st);                   // nothing of this call still writes the chunks
+      return e;
+    }
+  return cudaSuccess;
 }
 
 cudaError_t smem_limit_once(const void *kernel, int bytes) {
@@ -401,6 +514,11 @@ extern "C" int adga_destroy(adga_handle *h) {
   if (h->nfock_d) cudaFree(h->nfock_d);
   if (h->vq_extra) cudaFree(h->vq_extra);
   tan_free(h);
+  if (h->scr) cudaFree(h->scr);
+  if (h->stage) cudaFreeHost(h->stage);
+  for (cudaEvent_t e : h->events) cudaEventDestroy(e);
+  for (cudaEvent_t e : h->stage_ev)
+    if (e) cudaEventDestroy(e);
   if (h->qidx_h) cudaFreeHost(h->qidx_h);
   if (h->e0) cudaEventDestroy(h->e0);
   if (h->e1) cudaEventDestroy(h->e1);
@@ -531,13 +649,12 @@ extern "C" int adga_vertex_transform(adga_handle *h, int iwb, int vertex_type, i
   if (!h || !chi_loc_dens || !chi_loc_magn) return ADGA_EINVAL;
   const size_t n = (size_t)h->c.N * h->c.N;
   z64 *tmp = nullptr;
-  if (cudaMalloc(&tmp, 2 * n * sizeof(z64)) != cudaSuccess) return fail(h, ADGA_ENOMEM, "transform output");
+  if (!scratch_parts(h, {{&tmp, 2 * n}})) return fail(h, ADGA_ENOMEM, "transform output");
   int r = vertex_g4(h, iwb, vertex_type, iwfmax_g4, nineq, ndims, g4_dens, g4_magn, tmp, tmp + n);
-  if (!r && (cudaMemcpyAsync(chi_loc_dens, tmp, n * sizeof(z64), cudaMemcpyDeviceToHost, h->st) != cudaSuccess ||
-             cudaMemcpyAsync(chi_loc_magn, tmp + n, n * sizeof(z64), cudaMemcpyDeviceToHost, h->st) != cudaSuccess ||
+  if (!r && (download(h, chi_loc_dens, tmp, n * sizeof(z64)) != cudaSuccess ||
+             download(h, chi_loc_magn, tmp + n, n * sizeof(z64)) != cudaSuccess ||
              cudaStreamSynchronize(h->st) != cudaSuccess))
     r = fail(h, ADGA_ECUDA, "transform download");
-  cudaFree(tmp);
   return r;
 }
 
@@ -1192,8 +1309,9 @@ static int run_batch(adga_handle *h, int iwb, int np, int off, int prec, int *st
   cudaStream_t st = h->st;
   const size_t N = c.N, R = c.R;
   const int NB = prec == ADGA_FP64 ? 64 : h->NB;
-  cudaEvent_t ev[6];
-  for (int i = 0; i < 6; ++i) cudaEventCreate(&ev[i]);
+  const int nst = (int)((N + NB - 1) / NB);
+  cudaEvent_t *ev = batch_events(h, 6 + 2 * (size_t)nst), *tev = ev + 6;
+  if (!ev) return fail(h, ADGA_ECUDA, "timing events");
   CK(cudaMemcpyAsync(h->qidx_d, h->qidx_h, sizeof(int) * np, cudaMemcpyHostToDevice, st));
   cudaEventRecord(ev[0], st);
   CK(launch_chi0(c, iwb, h->qidx_d, np, h->chi0_all, h->nnu_all, st));
@@ -1209,11 +1327,8 @@ static int run_batch(adga_handle *h, int iwb, int np, int off, int prec, int *st
   int mixed_fail = 0, iters = 0;
   double worst = 0.0;
   std::vector<int> fallback;
-  const int nst = (int)((N + NB - 1) / NB);
-  std::vector<cudaEvent_t> tev(2 * nst);
-  for (auto &x : tev) cudaEventCreate(&x);
   TrailTiming tt;
-  tt.ev = tev.data();
+  tt.ev = tev;
   if (prec == ADGA_FP64) {
     z64 *T = (z64 *)h->Tm;
     CK(launch_bse_build<z64>(c, np, chi0q, h->c0inv, h->Frow_d, h->Frow_m, h->opg_d, h->opg_m, T,
@@ -1352,12 +1467,10 @@ static int run_batch(adga_handle *h, int iwb, int np, int off, int prec, int *st
   stage_ms(h, &h->stats.ms_lu, ev[2], ev[3]);
   stage_ms(h, &h->stats.ms_post, ev[3], ev[4]);
   stage_ms(h, &h->stats.ms_eom, ev[4], ev[5]);
-  for (int i = 0; i < 6; ++i) cudaEventDestroy(ev[i]);
   for (int i = 0; i < tt.n; ++i) stage_ms(h, &h->stats.ms_trail, tev[2 * i], tev[2 * i + 1]);
   h->stats.trail_launches += tt.n;
   h->stats.trail_gflop += tt.gflop;
   h->stats.trail_gbytes += tt.gbytes;
-  for (auto &x : tev) cudaEventDestroy(x);
   for (int p = 0; p < np; ++p) {
     int a = info[2 * p], b = info[2 * p + 1];
     int s = a ? a : b;
@@ -1655,7 +1768,7 @@ extern "C" int adga_get_tangent_outputs(adga_handle *h, int dir, const adga_outp
   CK(launch_mirror_sigma(c, t->sigma_nl, c.nkp_eom, st));
   const size_t np = h->last_npts;
 #define TDN(dst, src, n) \
-  if (dst) CK(cudaMemcpyAsync(dst, src, sizeof(z64) * (n), cudaMemcpyDeviceToHost, st))
+  if (dst) CK(download(h, dst, src, sizeof(z64) * (n)))
   if (np && t->chi_qw_d) {
     TDN(o->chi_qw_dens, t->chi_qw_d, np * h->nd4);
     TDN(o->chi_qw_magn, t->chi_qw_m, np * h->nd4);
@@ -1684,10 +1797,9 @@ extern "C" int adga_post_loop(adga_handle *h, adga_z *sigma_sum, adga_z *sigma_l
   if (c.nd > GINV_MAXND_HOST) return fail(h, ADGA_EINVAL, "post_loop: ndim above 8");
   const size_t ns = (size_t)c.nd2 * 2 * c.iwf * c.nkp_eom, ngl = (size_t)2 * c.iwmax * c.nd2;
   const size_t nsl = (size_t)c.nd2 * 2 * c.iwf, nnk = (size_t)c.nkp_eom * c.nd2;
-  z64 *buf = nullptr;
-  const size_t total = ns + nsl + ngl + nnk + c.nd;
-  if (cudaMalloc(&buf, total * sizeof(z64)) != cudaSuccess) return fail(h, ADGA_ENOMEM, "post_loop buffers");
-  z64 *sig = buf, *sl = sig + ns, *gl = sl + nsl, *nk = gl + ngl, *n = nk + nnk;
+  z64 *sig, *sl, *gl, *nk, *n;
+  if (!scratch_parts(h, {{&sig, ns}, {&sl, nsl}, {&gl, ngl}, {&nk, nnk}, {&n, (size_t)c.nd}}))
+    return fail(h, ADGA_ENOMEM, "post_loop buffers");
   cudaError_t e;
   if (sigma_sum) {
     e = cudaMemcpyAsync(sig, sigma_sum, ns * sizeof(z64), cudaMemcpyHostToDevice, st);
@@ -1700,7 +1812,7 @@ extern "C" int adga_post_loop(adga_handle *h, adga_z *sigma_sum, adga_z *sigma_l
     e = launch_post_loop(c, c.keom, sig, sigma_loc ? sl : nullptr, gloc ? gl : nullptr,
                          (n_dga_k || n_dga) ? nk : nullptr, n_dga ? n : nullptr, st);
 #define PDN(dst, src, cnt) \
-  if (e == cudaSuccess && dst) e = cudaMemcpyAsync(dst, src, (cnt) * sizeof(z64), cudaMemcpyDeviceToHost, st)
+  if (e == cudaSuccess && dst) e = download(h, dst, src, (cnt) * sizeof(z64))
   PDN(sigma_sum, sig, ns);
   PDN(sigma_loc, sl, nsl);
   PDN(gloc, gl, ngl);
@@ -1708,7 +1820,6 @@ extern "C" int adga_post_loop(adga_handle *h, adga_z *sigma_sum, adga_z *sigma_l
   PDN(n_dga, n, (size_t)c.nd);
 #undef PDN
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(buf);
   if (e != cudaSuccess) return fail(h, ADGA_ECUDA, std::string("post_loop: ") + cudaGetErrorString(e));
   return 0;
 }
@@ -1721,7 +1832,7 @@ extern "C" int adga_get_outputs(adga_handle *h, const adga_outputs *o) {
   CK(launch_mirror_sigma(c, h->sigma_nl, c.nkp_eom, st));
   const size_t np = h->last_npts;
 #define DN(dst, src, n) \
-  if (dst) CK(cudaMemcpyAsync(dst, src, sizeof(z64) * (n), cudaMemcpyDeviceToHost, st))
+  if (dst) CK(download(h, dst, src, sizeof(z64) * (n)))
   if (np) {
     DN(o->chi_qw_dens, h->chi_qw_d, np * h->nd4);
     DN(o->chi_qw_magn, h->chi_qw_m, np * h->nd4);
@@ -1819,9 +1930,8 @@ extern "C" int adga_bse_point(adga_handle *h, int iq, int iwb, int precision, ad
   r = ensure_work(h, precision, 1);
   if (r) return r;
   z64 *scr = nullptr;
-  std::vector<void *> tmp;
   // per-point outputs: the point's slot and one scratch slot for a re-solve
-  if (!alloc_into(h, scr, (size_t)6 * h->nd4, tmp)) return fail(h, ADGA_ENOMEM, "scratch");
+  if (!scratch_parts(h, {{&scr, (size_t)6 * h->nd4}})) return fail(h, ADGA_ENOMEM, "scratch");
   h->qidx_h[0] = iq - 1;
   int st_info[2] = {0, 0};
   memset(&h->stats, 0, sizeof(h->stats));
@@ -1842,7 +1952,6 @@ extern "C" int adga_bse_point(adga_handle *h, int iq, int iwb, int precision, ad
     if (gammaqd) cudaMemcpyAsync(gammaqd, h->gq, sizeof(z64) * n, cudaMemcpyDeviceToHost, h->st);
     if (cudaStreamSynchronize(h->st) != cudaSuccess) r = fail(h, ADGA_ECUDA, "copy-out");
   }
-  free_list(tmp);
   if (lu_info) *lu_info = st_info[0];
   return r;
 }
@@ -1851,14 +1960,10 @@ extern "C" int adga_calc_chi_qw(adga_handle *h, adga_z *chi_qw, const adga_z *in
                                 const adga_z *chi0_sum) {
   if (!h || !chi_qw || !interm3 || !chi0_sum) return ADGA_EINVAL;
   const DevCtx &c = h->c;
-  std::vector<void *> tmp;
   z64 *dchi, *dim3_, *dc0;
   const size_t nI = (size_t)c.nd2 * c.N, nC = (size_t)h->nd4 * 2 * c.iwf;
-  if (!alloc_into(h, dchi, h->nd4, tmp) || !alloc_into(h, dim3_, nI, tmp) ||
-      !alloc_into(h, dc0, nC, tmp)) {
-    free_list(tmp);
+  if (!scratch_parts(h, {{&dchi, (size_t)h->nd4}, {&dim3_, nI}, {&dc0, nC}}))
     return fail(h, ADGA_ENOMEM, "calc_chi_qw buffers");
-  }
   cudaStream_t st = h->st;
   cudaMemcpyAsync(dchi, chi_qw, sizeof(z64) * h->nd4, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(dim3_, interm3, sizeof(z64) * nI, cudaMemcpyHostToDevice, st);
@@ -1866,7 +1971,6 @@ extern "C" int adga_calc_chi_qw(adga_handle *h, adga_z *chi_qw, const adga_z *in
   cudaError_t e = launch_calc_chi_qw(c, dchi, dim3_, dc0, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(chi_qw, dchi, sizeof(z64) * h->nd4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  free_list(tmp);
   if (e != cudaSuccess) return fail(h, ADGA_ECUDA, cudaGetErrorString(e));
   return 0;
 }
@@ -1881,14 +1985,10 @@ extern "C" int adga_calc_eom_dynamic(adga_handle *h, const adga_z *etaqd, const 
   int r = ensure_work(h, prec, 1);
   if (r) return r;
   const size_t n = (size_t)c.nd2 * c.N, ns = (size_t)c.nd2 * 2 * c.iwf * c.nkp_eom;
-  std::vector<void *> tmp;
   z64 *X, *scr, *chi0z, *opz, *sig;
-  if (!alloc_into(h, X, 2 * n, tmp) || !alloc_into(h, scr, 2 * h->nd4, tmp) ||
-      !alloc_into(h, chi0z, (size_t)h->nd4 * 2 * c.iwf, tmp) || !alloc_into(h, opz, n, tmp) ||
-      !alloc_into(h, sig, ns, tmp)) {
-    free_list(tmp);
+  if (!scratch_parts(h, {{&X, 2 * n}, {&scr, 2 * (size_t)h->nd4}, {&chi0z, (size_t)h->nd4 * 2 * c.iwf}, {&opz, n},
+                         {&sig, ns}}))
     return fail(h, ADGA_ENOMEM, "eom buffers");
-  }
   cudaStream_t st = h->st;
   // Feed eta through the post kernel as X = eta^T with zero (1+gamma): it
   // rebuilds eta and forms m_tot with the reference's coefficients.
@@ -1909,7 +2009,7 @@ extern "C" int adga_calc_eom_dynamic(adga_handle *h, const adga_z *etaqd, const 
   const z64 *gwd = opz;
   if (e == cudaSuccess && c.vq) {
     int rl = ensure_local(h, iwb);
-    if (rl) { free_list(tmp); return rl; }
+    if (rl) return rl;
     gwd = h->gam_d;
   }
   if (e == cudaSuccess)
@@ -1917,9 +2017,8 @@ extern "C" int adga_calc_eom_dynamic(adga_handle *h, const adga_z *etaqd, const 
                     h->mtot, h->etad, h->etam, h->qidx_d, st);
   if (e == cudaSuccess) e = launch_eom_dynamic(c, iwb, h->qidx_d, 1, h->mtot, sig, st);
   if (e == cudaSuccess) e = launch_mirror_sigma(c, sig, c.nkp_eom, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(sigma_nl, sig, sizeof(z64) * ns, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = download(h, sigma_nl, sig, sizeof(z64) * ns);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  free_list(tmp);
   if (e != cudaSuccess) return fail(h, ADGA_ECUDA, cudaGetErrorString(e));
   return 0;
 }
@@ -1929,19 +2028,14 @@ extern "C" int adga_calc_eom_dmft(adga_handle *h, const adga_z *gammawd, int iwb
   DevCtx &c = h->c;
   if (iwb < -c.iwb || iwb > c.iwb) return ADGA_EINVAL;
   const size_t n = (size_t)c.nd2 * c.N, ns = (size_t)c.nd2 * 2 * c.iwf;
-  std::vector<void *> tmp;
   z64 *g, *s;
-  if (!alloc_into(h, g, n, tmp) || !alloc_into(h, s, ns, tmp)) {
-    free_list(tmp);
-    return fail(h, ADGA_ENOMEM, "eom_dmft buffers");
-  }
+  if (!scratch_parts(h, {{&g, n}, {&s, ns}})) return fail(h, ADGA_ENOMEM, "eom_dmft buffers");
   cudaStream_t st = h->st;
   cudaError_t e = cudaMemcpyAsync(g, gammawd, sizeof(z64) * n, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(s, sigma_dmft, sizeof(z64) * ns, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = launch_eom_dmft(c, iwb, g, s, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(sigma_dmft, s, sizeof(z64) * ns, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  free_list(tmp);
   if (e != cudaSuccess) return fail(h, ADGA_ECUDA, cudaGetErrorString(e));
   return 0;
 }
@@ -1951,15 +2045,13 @@ extern "C" int adga_calc_eom_static(adga_handle *h, int iq, adga_z *sigma_dmft) 
   if (iq != 1) return 0;       // the local Hartree term only enters at q = 1
   DevCtx &c = h->c;
   const size_t ns = (size_t)c.nd2 * 2 * c.iwf;
-  std::vector<void *> tmp;
   z64 *s;
-  if (!alloc_into(h, s, ns, tmp)) return fail(h, ADGA_ENOMEM, "eom_static buffers");
+  if (!scratch_parts(h, {{&s, ns}})) return fail(h, ADGA_ENOMEM, "eom_static buffers");
   cudaStream_t st = h->st;
   cudaError_t e = cudaMemcpyAsync(s, sigma_dmft, sizeof(z64) * ns, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = launch_eom_static(c, s, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(sigma_dmft, s, sizeof(z64) * ns, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  free_list(tmp);
   if (e != cudaSuccess) return fail(h, ADGA_ECUDA, cudaGetErrorString(e));
   return 0;
 }
@@ -1970,38 +2062,31 @@ extern "C" int adga_calc_eom_static(adga_handle *h, int iq, adga_z *sigma_dmft) 
 extern "C" int adga_inverse_matrix_z(adga_z *M, int n, int *ierr, char *erstr) {
   if (!M || n < 1 || n > 4096) return ADGA_EINVAL;
   const int NB = 64, nsteps = (n + NB - 1) / NB;
-  const size_t strideM = (size_t)n * 2 * n;
-  z64 *T = nullptr, *Li = nullptr, *Ui = nullptr;
-  int *ip = nullptr, *inf = nullptr, *rm = nullptr;
+  const size_t nn = (size_t)n * n, strideM = 2 * nn, nblk = (size_t)nsteps * NB * NB;
+  // one allocation: the matrix with the identity beside it, the block inverses, pivots, info and row map
+  const size_t elems = strideM + 2 * nblk, ints = (size_t)n + 1 + RMAP_STRIDE;
+  char *buf = nullptr;
   cudaStream_t st;
   if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return ADGA_ECUDA;
   int rc = 0;
-  std::vector<adga_z> aug((size_t)n * 2 * n);
-  memcpy(aug.data(), M, sizeof(adga_z) * n * n);
-  for (int j = 0; j < n; ++j)
-    for (int i = 0; i < n; ++i) {
-      adga_z v = {i == j ? 1.0 : 0.0, 0.0};
-      aug[(size_t)n * n + i + (size_t)j * n] = v;
-    }
-  if (cudaMalloc(&T, sizeof(z64) * strideM) != cudaSuccess ||
-      cudaMalloc(&Li, sizeof(z64) * nsteps * NB * NB) != cudaSuccess ||
-      cudaMalloc(&Ui, sizeof(z64) * nsteps * NB * NB) != cudaSuccess ||
-      cudaMalloc(&ip, sizeof(int) * n) != cudaSuccess || cudaMalloc(&inf, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&rm, sizeof(int) * RMAP_STRIDE) != cudaSuccess) {
+  if (cudaMalloc(&buf, elems * sizeof(z64) + ints * sizeof(int)) != cudaSuccess) {
     rc = ADGA_ENOMEM;
   } else {
+    z64 *T = (z64 *)buf, *Li = T + strideM, *Ui = Li + nblk;
+    int *ip = (int *)(Ui + nblk), *inf = ip + n, *rm = inf + 1;
     LUBatch lb{n, 2 * n, 1, NB, strideM, ip, inf, Li, Ui, rm};
     int info = 0;
-    cudaError_t e = cudaMemcpyAsync(T, aug.data(), sizeof(z64) * strideM, cudaMemcpyHostToDevice, st);
+    cudaError_t e = cudaMemcpyAsync(T, M, sizeof(z64) * nn, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = launch_identity(n, T + nn, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(inf, 0, sizeof(int), st);
     if (lu_small_supported(n, n)) {
       if (e == cudaSuccess) e = lu_small_solve(T, strideM, n, n, 1, inf, st);
     } else {
       if (e == cudaSuccess) e = lu_factor<z64>(T, lb, false, nullptr, nullptr, st);
-      if (e == cudaSuccess) e = lu_backsolve<z64>(T, lb, T + (size_t)n * n, strideM, n, n, st);
+      if (e == cudaSuccess) e = lu_backsolve<z64>(T, lb, T + nn, strideM, n, n, st);
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(&info, inf, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(M, T + (size_t)n * n, sizeof(z64) * n * n, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(M, T + nn, sizeof(z64) * nn, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = ADGA_ECUDA;
     if (ierr) *ierr = info;
@@ -2011,7 +2096,7 @@ extern "C" int adga_inverse_matrix_z(adga_z *M, int n, int *ierr, char *erstr) {
     }
     if (rc == 0 && info) rc = info;
   }
-  cudaFree(T); cudaFree(Li); cudaFree(Ui); cudaFree(ip); cudaFree(inf); cudaFree(rm);
+  cudaFree(buf);
   cudaStreamDestroy(st);
   return rc;
 }

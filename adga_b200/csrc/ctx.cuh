@@ -133,6 +133,7 @@ cudaError_t launch_eom_dynamic(const DevCtx &c, int iwb, const int *qidx, int np
                                const z64 *mtot, z64 *sigma_nl, cudaStream_t st);
 
 // k_refine.cu
+cudaError_t launch_identity(int n, z64 *E, cudaStream_t st);
 cudaError_t launch_init_x(const z32 *T32, size_t strideM, int N, int R, int nmat, z64 *X, cudaStream_t st);
 // rnorm (nullable): per-matrix max |re| + |im| of the FP64 residual, atomicMax on the bit patterns;
 // Bpt (nullable): per-point right-hand sides in X's layout instead of (1+gamma^w) (tangent solves)

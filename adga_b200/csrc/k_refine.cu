@@ -19,6 +19,16 @@ cudaError_t launch_resid_z64(const DevCtx &c, int npts, const z64 *XD, const z64
                              const z64 *opg_m, z32 *V, const z64 *extra_d, unsigned long long *rnorm,
                              const z64 *Bpt, cudaStream_t st);
 
+// the n x n identity
+__global__ void k_identity(int n, z64 *E) {
+  const size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (idx < (size_t)n * n) E[idx] = make_double2(idx % n == idx / n ? 1.0 : 0.0, 0.0);
+}
+cudaError_t launch_identity(int n, z64 *E, cudaStream_t st) {
+  k_identity<<<cdiv_u((size_t)n * n, 256), 256, 0, st>>>(n, E);
+  return ADGA_LAUNCH_CHECK();
+}
+
 // X64 = up(Y32) from the RHS columns of the FP32 factorised matrices
 __global__ void k_init_x(const z32 *T32, size_t strideM, int N, int R, int nmat, z64 *X) {
   size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
