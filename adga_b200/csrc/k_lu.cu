@@ -13,32 +13,36 @@
 //                BF16x3 kernel of the mixed path).
 // Pivot choice follows izamax: the largest |re|+|im|, the lowest row on ties.
 #include "lu.cuh"
+#include "zgemm.cuh"
 #include <algorithm>
 #include <climits>
 
 
 // ---------------------------------------------------------------------------
 // Panel factorisation, one CTA per matrix: SW-column sub-panels live in
-// registers (thread t owns rows J + t + q nt), and the rest of the panel takes
+// registers (thread t holds rows J + t + q nt), and the rest of the panel takes
 // their interchanges, triangular solve and rank-SW update from global memory.
 //
-// Bound by the serial chain of a column: the pivot search is three integer
-// warp reductions over the bit pattern of |re|+|im| (high word, low word, then
-// the lowest row), every warp's candidate row is put in shared memory beside
-// its key before the one barrier of the column, and after it every warp
-// reduces the candidates itself, so that neither a second reduction stage nor
-// a row broadcast needs another barrier.  The buffers alternate with the
-// column's parity.  Sub-panels of 16 columns where one row per thread fits
-// (rows <= 512: half the passes over the rest of the panel), else of 8 and less.
-// With double-precision shuffles, three barriers a column and a serially
-// composed interchange map: 137 us for a 40 x 40 panel, 417 us for 1016 x 64,
-// 1799 us for 500 of them; this form: 66 us, 250 us and 1182 us.
+// Bound by the serial chain of a column on few rows, by the passes over the
+// panel on many.  The pivot search is three integer warp reductions over the
+// bit pattern of |re|+|im| (high word, low word, then the lowest row), every
+// warp's candidate row is put in shared memory beside its key before the one
+// barrier of the column, and after it every warp reduces the candidates itself,
+// so that neither a second reduction stage nor a row broadcast needs another
+// barrier; the buffers alternate with the column's parity.  Rows keep their
+// registers: an interchange only swaps the positions they stand for.  The next
+// column is updated and searched before the rest of the row.  Sub-panels of 16
+// columns where one row per thread fits (rows <= 512: half the passes over the
+// rest of the panel), else of 8 and less.
+// With double-precision shuffles, three barriers a column, rows moved through
+// shared memory and a serially composed interchange map: 137 us for a 40 x 40
+// panel, 310 us for 357 x 64, 417 us for 1016 x 64, 1799 us for 500 of those;
+// this form: 40 us, 110 us, 250 us and 1193 us.
 // ---------------------------------------------------------------------------
 template <typename T, int SW> struct PanelShared {
   unsigned long long key[2][32];
   int row[2][32];
-  T cand[2][32][SW];           // each warp's candidate row
-  T crow[2][SW];               // the row at the diagonal
+  T cand[2][32][SW];           // each warp's candidate row, from the column on
   T Lss[SW * SW];
   int piv[SW], dst[2 * SW], src[2 * SW], cnt;
 };
@@ -63,36 +67,39 @@ __device__ __forceinline__ z64 crcp_scaled(z64 z) {
 }
 __device__ __forceinline__ z32 crcp_scaled(z32 z) { return crcp(z); }
 
-// One column CC of the register-resident sub-panel.  CC is a compile-time
-// constant so that every index into the register array is static.
+// the warp's candidate for column CC: the row with the largest key, put beside the key
 template <typename T, int RPT, int SW, int CC>
-__device__ __forceinline__ void panel_column(T (&a)[RPT][SW], PanelShared<T, SW> &S, int J, int N, int c0, int sw,
-                                             int t, int nt, int *ipiv, int &info) {
+__device__ __forceinline__ void panel_search(const T (&a)[RPT][SW], const int (&pos)[RPT], PanelShared<T, SW> &S,
+                                             int N, int col, unsigned long long &key, int &row) {
+  key = 0;
+  row = INT_MAX;
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    // 1 + the bits of a non-negative number order like the number; NaN is never a pivot
+    unsigned long long k = (unsigned long long)__double_as_longlong((double)cabs1(a[q][CC]));
+    k = (pos[q] >= col && pos[q] < N && k <= 0x7ff0000000000000ULL) ? k + 1 : 0;
+    if (k > key || (k == key && k && pos[q] < row)) { key = k; row = pos[q]; }
+  }
+  warp_argmax(key, row);
+}
+
+// One column CC of the register-resident sub-panel.  CC is a compile-time
+// constant so that every index into the register array is static.  Rows do not
+// move: pos is the row of the matrix that a register row stands for, and an
+// interchange swaps two positions.  The next column is updated and searched
+// before the rest of the row.
+template <typename T, int RPT, int SW, int CC>
+__device__ __forceinline__ void panel_column(T (&a)[RPT][SW], int (&pos)[RPT], PanelShared<T, SW> &S, int N, int c0,
+                                             int sw, int t, int nt, int *ipiv, int &info, unsigned long long &key,
+                                             int &row) {
   if (CC >= sw) return;
   const int lane = t & 31, warp = t >> 5, nw = nt >> 5, par = CC & 1;
   const int col = c0 + CC;
-  unsigned long long key = 0;
-  int row = INT_MAX;
 #pragma unroll
-  for (int q = 0; q < RPT; ++q) {
-    const int r = J + t + q * nt;
-    const double v = (double)cabs1(a[q][CC]);
-    // 1 + the bits of a non-negative number order like the number; NaN is never a pivot
-    const unsigned long long k = (r >= col && r < N && v == v) ? (unsigned long long)__double_as_longlong(v) + 1 : 0;
-    if (k > key) { key = k; row = r; }
-  }
-  const int mine = row;
-  warp_argmax(key, row);
+  for (int q = 0; q < RPT; ++q)
+    if (key && pos[q] == row)
 #pragma unroll
-  for (int q = 0; q < RPT; ++q) {
-    const int r = J + t + q * nt;
-    if (key && r == row && mine == row)
-#pragma unroll
-      for (int c2 = 0; c2 < SW; ++c2) S.cand[par][warp][c2] = a[q][c2];
-    if (r == col)
-#pragma unroll
-      for (int c2 = 0; c2 < SW; ++c2) S.crow[par][c2] = a[q][c2];
-  }
+      for (int c2 = CC; c2 < SW; ++c2) S.cand[par][warp][c2] = a[q][c2];
   if (lane == 0) { S.key[par][warp] = key; S.row[par][warp] = row; }
   __syncthreads();
   unsigned long long k2 = lane < nw ? S.key[par][lane] : 0;
@@ -100,43 +107,52 @@ __device__ __forceinline__ void panel_column(T (&a)[RPT][SW], PanelShared<T, SW>
   const int rl = p;
   warp_argmax(k2, p);
   const unsigned who = __ballot_sync(0xffffffffu, k2 && rl == p && lane < nw);
-  const T *prow = who ? S.cand[par][__ffs(who) - 1] : S.crow[par];
-  if (!who) p = col;                       // no eligible row (all NaN)
-  const T piv = prow[CC];
-  const bool zero = piv.x == 0 && piv.y == 0;
-  if (zero && info == 0) info = col + 1;
-  const T rcp = zero ? czero<T>() : crcp_scaled(piv);
-  if (p != col) {
-#pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const int r = J + t + q * nt;
-      if (r == col)
-#pragma unroll
-        for (int c2 = 0; c2 < SW; ++c2) a[q][c2] = prow[c2];
-      else if (r == p)
-#pragma unroll
-        for (int c2 = 0; c2 < SW; ++c2) a[q][c2] = S.crow[par][c2];
-    }
-  }
+  T rcp = czero<T>();
+  const T *prow = S.cand[par][who ? __ffs(who) - 1 : 0];
+  const bool zero = k2 <= 1;               // the largest |re|+|im| is zero, or no row is eligible (all NaN)
+  if (!who) p = col;
+  if (k2 == 1 && info == 0) info = col + 1;
+  if (!zero) rcp = crcp_scaled(prow[CC]);
+  T l[RPT];
 #pragma unroll
   for (int q = 0; q < RPT; ++q) {
-    if (J + t + q * nt > col) {            // rows past N hold zeros
-      if (!zero) a[q][CC] = cmul(a[q][CC], rcp);
+    pos[q] = pos[q] == p ? col : pos[q] == col ? p : pos[q];
+    const bool below = pos[q] > col && pos[q] < N;
+    if (below && !zero) a[q][CC] = cmul(a[q][CC], rcp);
+    l[q] = below && who ? a[q][CC] : czero<T>();
+  }
+  if (CC + 1 < SW) {
+    const T u = prow[CC + 1 < SW ? CC + 1 : CC];
 #pragma unroll
-      for (int c2 = CC + 1; c2 < SW; ++c2) cfms(a[q][c2], a[q][CC], prow[c2]);
-    }
+    for (int q = 0; q < RPT; ++q) cfms(a[q][CC + 1 < SW ? CC + 1 : CC], l[q], u);
+    panel_search<T, RPT, SW, (CC + 1 < SW ? CC + 1 : CC)>(a, pos, S, N, col + 1, key, row);
+  }
+#pragma unroll
+  for (int c2 = CC + 2; c2 < SW; ++c2) {
+    const T u = prow[c2];
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) cfms(a[q][c2], l[q], u);
   }
   if (t == 0) { S.piv[CC] = p; ipiv[col] = p; }
 }
 
 template <typename T, int RPT, int SW, int CC>
-__device__ __forceinline__ void panel_columns(T (&a)[RPT][SW], PanelShared<T, SW> &S, int J, int N, int c0, int sw,
-                                              int t, int nt, int *ipiv, int &info) {
+__device__ __forceinline__ void panel_columns(T (&a)[RPT][SW], int (&pos)[RPT], PanelShared<T, SW> &S, int N, int c0,
+                                              int sw, int t, int nt, int *ipiv, int &info, unsigned long long &key,
+                                              int &row) {
   if constexpr (CC < SW) {
-    panel_column<T, RPT, SW, CC>(a, S, J, N, c0, sw, t, nt, ipiv, info);
-    panel_columns<T, RPT, SW, CC + 1>(a, S, J, N, c0, sw, t, nt, ipiv, info);
+    panel_column<T, RPT, SW, CC>(a, pos, S, N, c0, sw, t, nt, ipiv, info, key, row);
+    panel_columns<T, RPT, SW, CC + 1>(a, pos, S, N, c0, sw, t, nt, ipiv, info, key, row);
   }
 }
+
+// One row per thread (rows <= 512): the rank-16 update of the rest of the panel on the FP64 tensor cores, whose
+// operands a warp reads once per 8 x 8 tile (a thread's row times broadcast U entries is bound by the shared-
+// memory reads: 46k against 30k clocks for the first update at 357 rows).  More rows per thread: their update is
+// bound by the memory passes, where a thread's own rows measured better (1016 rows: 250 against 278 us a panel).
+template <typename T, int RPT> constexpr bool panel_mma() { return sizeof(T) == sizeof(z64) && RPT == 1; }
+// stride of the staged multipliers: 2 mod 8 elements, conflict-free fragment reads (lane = 4 row + k)
+__host__ __device__ inline int panel_lr(int rows) { return (rows + 7) / 8 * 8 + 2; }
 
 template <typename T, int RPT, int SW, int NTMAX>
 __global__ void __launch_bounds__(NTMAX, 1)
@@ -148,6 +164,8 @@ k_panel(T *M, size_t strideM, int N, int J, int jb, int *ipiv_all, int *info_all
   __shared__ PanelShared<T, SW> S;
   extern __shared__ __align__(16) unsigned char panel_dyn[];
   T *Gs = reinterpret_cast<T *>(panel_dyn);        // [jb - sw columns][2 SW]: moved rows, then U in the first SW
+  T *Ls = Gs + 64 * 2 * SW;                        // panel_mma: the sub-panel's multipliers, [SW][LR]
+  const int LR = panel_lr(N - J);
   int info = info_all[b];
   T a[RPT][SW];
 
@@ -161,11 +179,16 @@ k_panel(T *M, size_t strideM, int N, int J, int jb, int *ipiv_all, int *info_all
       for (int cc = 0; cc < SW; ++cc)
         a[q][cc] = (r >= c0 && r < N && cc < sw) ? A[r + (size_t)(c0 + cc) * N] : czero<T>();
     }
-    panel_columns<T, RPT, SW, 0>(a, S, J, N, c0, sw, t, nt, ipiv, info);
+    int pos[RPT], row;
+    unsigned long long key;
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) pos[q] = J + t + q * nt;
+    panel_search<T, RPT, SW, 0>(a, pos, S, N, c0, key, row);
+    panel_columns<T, RPT, SW, 0>(a, pos, S, N, c0, sw, t, nt, ipiv, info, key, row);
     // the sub-panel back to the matrix; its L block for the solve below
 #pragma unroll
     for (int q = 0; q < RPT; ++q) {
-      const int r = J + t + q * nt;
+      const int r = pos[q];
       if (r >= c0 && r < N) {
 #pragma unroll
         for (int cc = 0; cc < SW; ++cc)
@@ -174,6 +197,9 @@ k_panel(T *M, size_t strideM, int N, int J, int jb, int *ipiv_all, int *info_all
         if (i < SW)
 #pragma unroll
           for (int cc = 0; cc < SW; ++cc) S.Lss[i + cc * SW] = a[q][cc];
+        else if (panel_mma<T, RPT>())
+#pragma unroll
+          for (int cc = 0; cc < SW; ++cc) Ls[(size_t)cc * LR + r - J] = a[q][cc];
       }
     }
     if (jb == sw) break;                           // the panel is this sub-panel
@@ -244,23 +270,71 @@ k_panel(T *M, size_t strideM, int N, int J, int jb, int *ipiv_all, int *info_all
       }
     }
     __syncthreads();
-    // rank-SW update of the rows below, right panel columns, in chunks of CW columns whose loads are
-    // all issued before their stores (a full sub-panel: sw == SW whenever columns are left)
-    if (nright > 0) {
-      constexpr int CW = sizeof(T) == 8 ? 4 : (RPT == 1 ? 4 : 2);
+    // rank-SW update of the rows below, right panel columns (a full sub-panel: sw == SW whenever columns
+    // are left)
+    if constexpr (panel_mma<T, RPT>()) {
+      // warps take 8-row tiles, eight columns at a time, on the FP64 tensor cores: C - L U with C as the
+      // accumulators' start
+      const int warp = t >> 5, lane = t & 31, kl = lane & 3, rl = lane >> 2;
       const T *U = Gs + s * 2 * SW;
-      T *arow = A + J + t + (size_t)(c0 + sw) * N;
+      for (int m0 = c0 + sw + 8 * warp; m0 < N; m0 += 8 * (nt >> 5)) {
+        const int r = m0 + rl;
+        z64 l[(SW + 3) / 4];
+#pragma unroll
+        for (int k = 0; k < (SW + 3) / 4; ++k)
+          l[k] = 4 * k + kl < SW && r < N ? Ls[(size_t)(4 * k + kl) * LR + r - J] : czero<z64>();
+        constexpr int NB = 2;                      // column tiles in flight
+        for (int n0 = 0; n0 < nright; n0 += 8 * NB) {
+          double re[NB][2], im[NB][2];
+#pragma unroll
+          for (int j = 0; j < NB; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int c = n0 + 8 * j + 2 * kl + e;
+              const z64 v = r < N && c < nright ? A[r + (size_t)(c0 + sw + c) * N] : czero<z64>();
+              re[j][e] = v.x;
+              im[j][e] = v.y;
+            }
+#pragma unroll
+          for (int k = 0; k < (SW + 3) / 4; ++k)
+#pragma unroll
+            for (int j = 0; j < NB; ++j) {
+              const int c = n0 + 8 * j + rl;
+              const z64 u = c < nright && 4 * k + kl < SW ? U[c * 2 * SW + 4 * k + kl] : czero<z64>();
+              zg::dmma(re[j], -l[k].x, u.x);
+              zg::dmma(im[j], -l[k].x, u.y);
+              zg::dmma(re[j], l[k].y, u.y);
+              zg::dmma(im[j], -l[k].y, u.x);
+            }
+#pragma unroll
+          for (int j = 0; j < NB; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int c = n0 + 8 * j + 2 * kl + e;
+              if (r < N && c < nright) A[r + (size_t)(c0 + sw + c) * N] = make_double2(re[j][e], im[j][e]);
+            }
+        }
+      }
+    } else if (nright > 0) {
+      // the thread's own rows, in chunks of CW columns whose loads are all issued before their stores
+      constexpr int CW = sizeof(T) == 8 ? 4 : 2;
+      const T *U = Gs + s * 2 * SW;
+      T *ar[RPT];
+      bool in[RPT];
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+        in[q] = pos[q] >= c0 + sw && pos[q] < N;
+        ar[q] = A + pos[q] + (size_t)(c0 + sw) * N;
+      }
 #pragma unroll 1
       for (int u0 = 0; u0 < nright; u0 += CW) {
         T v[RPT][CW];
 #pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-          const int r = J + t + q * nt;
-          if (r >= c0 + sw && r < N)
+        for (int q = 0; q < RPT; ++q)
+          if (in[q])
 #pragma unroll
             for (int j = 0; j < CW; ++j)
-              if (u0 + j < nright) v[q][j] = arow[q * nt + (size_t)(u0 + j) * N];
-        }
+              if (u0 + j < nright) v[q][j] = ar[q][(size_t)(u0 + j) * N];
 #pragma unroll
         for (int j = 0; j < CW; ++j)
 #pragma unroll
@@ -270,13 +344,11 @@ k_panel(T *M, size_t strideM, int N, int J, int jb, int *ipiv_all, int *info_all
             for (int q = 0; q < RPT; ++q) cfms(v[q][j], a[q][i], y);
           }
 #pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-          const int r = J + t + q * nt;
-          if (r >= c0 + sw && r < N)
+        for (int q = 0; q < RPT; ++q)
+          if (in[q])
 #pragma unroll
             for (int j = 0; j < CW; ++j)
-              if (u0 + j < nright) arow[q * nt + (size_t)(u0 + j) * N] = v[q][j];
-        }
+              if (u0 + j < nright) ar[q][(size_t)(u0 + j) * N] = v[q][j];
       }
     }
     __syncthreads();
@@ -1270,8 +1342,8 @@ template <typename T, int RPT, int SW, int NTMAX>
 static cudaError_t launch_panel_as(T *M, const LUBatch &lb, int J, int jb, cudaStream_t st) {
   const int rows = lb.N - J;
   const int nt = std::max(128, ((rows + RPT - 1) / RPT + 31) / 32 * 32);
-  const size_t dyn = sizeof(T) * (size_t)64 * 2 * SW;
-  smem_limit(k_panel<T, RPT, SW, NTMAX>, (int)dyn);
+  const size_t dyn = sizeof(T) * ((size_t)64 * 2 * SW + (panel_mma<T, RPT>() ? (size_t)SW * panel_lr(rows) : 0));
+  smem_limit(k_panel<T, RPT, SW, NTMAX>, 200 * 1024);
   k_panel<T, RPT, SW, NTMAX><<<lb.batch, nt, dyn, st>>>(M, lb.strideM, lb.N, J, jb, lb.ipiv, lb.info);
   return ADGA_LAUNCH_CHECK();
 }
@@ -1279,13 +1351,14 @@ static cudaError_t launch_panel_as(T *M, const LUBatch &lb, int J, int jb, cudaS
 template <typename T>
 static cudaError_t launch_panel(T *M, const LUBatch &lb, int J, int jb, cudaStream_t st) {
   const int rows = lb.N - J;
-  // rows x SW complex values fill the register file at 512 x 16, 1024 x 8, 2048 x 4 and 4096 x 2; wider
+  // rows x SW complex values fill the register file at 512 x 16, 1152 x 8, 2048 x 4 and 4096 x 2; wider
   // sub-panels halve the passes over the rest of the panel, spilled ones cost more than they save
-  // (one 64-column panel, us, as listed / with the next wider or narrower form: 1016 rows 255 / 301,
-  // 1080 rows 330 / 395, 1500 rows 418 / 428, 2000 rows 543 / 998, 4000 rows 2666 / 3839)
+  // (one 64-column panel, us, as listed against another form: 1016 rows 250 / 275 at three rows a thread,
+  // 1080 rows 276 / 337 at <2, 4>, 1500 rows 415 / 606 and 2000 rows 539 / 795 with the update on the
+  // tensor cores, 4000 rows 2700 / 3839 at <8, 4>)
   if (rows <= 512) return launch_panel_as<T, 1, 16, 512>(M, lb, J, jb, st);
   if (rows <= 1024) return launch_panel_as<T, 2, 8, 512>(M, lb, J, jb, st);
-  if (rows <= 1280) return launch_panel_as<T, 2, 4, 640>(M, lb, J, jb, st);
+  if (rows <= 1152) return launch_panel_as<T, 3, 8, 384>(M, lb, J, jb, st);
   if (rows <= 1536) return launch_panel_as<T, 2, 4, 768>(M, lb, J, jb, st);
   if (rows <= 2048) return launch_panel_as<T, 4, 4, 512>(M, lb, J, jb, st);
   if (rows <= 4096) return launch_panel_as<T, 8, 2, 512>(M, lb, J, jb, st);
