@@ -142,7 +142,7 @@ struct TanState {
 };
 // batch work and constants shared by the directions (they run one after another)
 struct TanWork {
-  z64 *zero_nd4 = nullptr, *zero_N = nullptr, *zero_gam = nullptr, *opg_scr = nullptr, *bub_scr = nullptr;
+  z64 *zero_nd4 = nullptr, *zero_N = nullptr, *zero_gam = nullptr, *bub_scr = nullptr;
   std::vector<void *> owned, work;
   int cap = 0;
   z64 *chi0_all = nullptr, *chi0_tmp = nullptr, *chi0q_big = nullptr, *zero_chi0 = nullptr;
@@ -761,8 +761,7 @@ static int ensure_local(adga_handle *h, int iwb) {
   if (!h->vd[w]) return fail(h, ADGA_ESTATE, "vertex of omega " + std::to_string(iwb) + " not set");
   int r = ensure_diag(h, iwb);
   if (r) return r;
-  CK(launch_local_F(h->c, h->vd[w], h->c0inv, h->Frow_d, h->st));
-  CK(launch_local_F(h->c, h->vm[w], h->c0inv, h->Frow_m, h->st));
+  CK(launch_local_F(h->c, h->vd[w], h->vm[w], h->c0inv, h->Frow_d, h->Frow_m, h->st));
   h->f32_iwb = INT_MIN;
   ++h->frow_gen;
   if (h->tl_d[w]) {
@@ -773,8 +772,7 @@ static int ensure_local(adga_handle *h, int iwb) {
     CK(launch_one_plus_gamma(h->c, h->gam_d, h->opg_d, h->st));
     CK(launch_one_plus_gamma(h->c, h->gam_m, h->opg_m, h->st));
   } else {
-    CK(launch_local_gamma(h->c, h->Frow_d, h->gam_d, h->opg_d, h->st));
-    CK(launch_local_gamma(h->c, h->Frow_m, h->gam_m, h->opg_m, h->st));
+    CK(launch_local_gamma(h->c, h->Frow_d, h->Frow_m, h->gam_d, h->gam_m, h->opg_d, h->opg_m, h->st));
   }
   h->loc_iwb = iwb;
   return 0;
@@ -932,7 +930,7 @@ static int tan_shared(adga_handle *h) {
   const size_t N = c.N, nd2 = c.nd2;
   auto &L = w->owned;
   if (!(alloc_into(h, w->zero_nd4, nd2 * nd2, L) && alloc_into(h, w->zero_N, N, L) &&
-        alloc_into(h, w->zero_gam, nd2 * N, L) && alloc_into(h, w->opg_scr, nd2 * N, L) &&
+        alloc_into(h, w->zero_gam, nd2 * N, L) &&
         alloc_into(h, w->bub_scr, nd2 * nd2, L)))
     return fail(h, ADGA_ENOMEM, "tangent constants");
   CK(cudaMemsetAsync(w->zero_nd4, 0, sizeof(z64) * nd2 * nd2, h->st));
@@ -1054,10 +1052,8 @@ static int tan_local(adga_handle *h, int d, int iwb) {
   t->loc_has = t->vd[w] != nullptr;
   if (t->loc_has) {
     // F~ = sym(chi_loc) chi0_loc^-1 - 1 is affine in chi_loc: dF~ = sym(dchi_loc) chi0_loc^-1
-    CK(launch_local_F(h->c, t->vd[w], h->c0inv, t->Fd, h->st, false));
-    CK(launch_local_F(h->c, t->vm[w], h->c0inv, t->Fm, h->st, false));
-    CK(launch_local_gamma(h->c, t->Fd, t->gd, h->tw->opg_scr, h->st));
-    CK(launch_local_gamma(h->c, t->Fm, t->gm, h->tw->opg_scr, h->st));
+    CK(launch_local_F(h->c, t->vd[w], t->vm[w], h->c0inv, t->Fd, t->Fm, h->st, false));
+    CK(launch_local_gamma(h->c, t->Fd, t->Fm, t->gd, t->gm, nullptr, nullptr, h->st));
   }
   t->loc_iwb = iwb;
   return 0;

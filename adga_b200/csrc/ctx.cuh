@@ -52,10 +52,12 @@ cudaError_t launch_kq_index(int nkpx, int nkpy, int nkpz, const int *k_sel, int 
                             const int *q_data, int nqp, int one_based, int *ind, cudaStream_t st);
 cudaError_t launch_local_diag(const DevCtx &c, int iwb, z64 *c0inv, z64 *c0w, z64 *bubloc_tmp,
                               cudaStream_t st);
-cudaError_t launch_local_F(const DevCtx &c, const z64 *chi_loc, const z64 *c0inv, z64 *Frow,
-                           cudaStream_t st, bool minus_one = true);
+cudaError_t launch_local_F(const DevCtx &c, const z64 *chi_d, const z64 *chi_m, const z64 *c0inv, z64 *Frow_d,
+                           z64 *Frow_m, cudaStream_t st, bool minus_one = true);
 cudaError_t launch_gtable_dot(const DevCtx &c, const z64 *dhk, z64 *gdot, cudaStream_t st);
-cudaError_t launch_local_gamma(const DevCtx &c, const z64 *Frow, z64 *gam, z64 *opg, cudaStream_t st);
+// opg_d / opg_m (1 + gamma^w) may be null
+cudaError_t launch_local_gamma(const DevCtx &c, const z64 *Frow_d, const z64 *Frow_m, z64 *gam_d, z64 *gam_m,
+                               z64 *opg_d, z64 *opg_m, cudaStream_t st);
 cudaError_t launch_chi_loc_update(const DevCtx &c, const z64 *gam_d, const z64 *gam_m,
                                   const z64 *c0w, const z64 *bubloc_tmp, z64 *chi_loc_d,
                                   z64 *chi_loc_m, z64 *bubble_loc, cudaStream_t st);

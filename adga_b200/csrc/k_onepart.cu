@@ -102,6 +102,15 @@ __device__ __forceinline__ z64 giw_at(const DevCtx &c, int n, int i) {
   return c.giw[(n + c.iwmax) + i * 2 * c.iwmax];
 }
 
+__device__ __forceinline__ z64 warp_sum(z64 v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  return v;
+}
+
 __global__ void k_local_diag(DevCtx c, int iwb, z64 *c0inv, z64 *c0w, z64 *bubloc_tmp) {
   int nd = c.nd, nd2 = c.nd2;
   int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -116,12 +125,17 @@ __global__ void k_local_diag(DevCtx c, int iwb, z64 *c0inv, z64 *c0w, z64 *bublo
     c0inv[tid] = cneg(crcp(t));
     // -beta*g_i*g_j      (get_chi0_loc)
     c0w[tid] = cmul(cscale(gi, -c.beta), gj);
-  } else if (tid < nsmall + nd2) {
-    int i2 = tid - nsmall;
+    return;
+  }
+  // the blocks after those: a warp per compound index, its lanes sharing the frequencies
+  const int i2 = ((int)blockIdx.x - (nsmall + 127) / 128) * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if ((int)blockIdx.x >= (nsmall + 127) / 128 && i2 < nd2) {
     int i = i2 / nd, j = i2 % nd;
     z64 s = czero<z64>();
-    for (int iwf = c.iwstart; iwf <= c.iwstop; ++iwf)
+    for (int iwf = c.iwstart + lane; iwf <= c.iwstop; iwf += 32)
       s = cadd(s, cmul(cscale(giw_at(c, iwf, i), -c.beta), giw_at(c, iwf - iwb, j)));
+    s = warp_sum(s);
+    if (lane) return;
     double b2 = c.beta * c.beta;
     // bubble_loc_tmp is diagonal in the compound index (zeroed by the launcher)
     bubloc_tmp[i2 + i2 * nd2] = make_double2(s.x / b2, s.y / b2);
@@ -130,16 +144,18 @@ __global__ void k_local_diag(DevCtx c, int iwb, z64 *c0inv, z64 *c0w, z64 *bublo
 
 cudaError_t launch_local_diag(const DevCtx &c, int iwb, z64 *c0inv, z64 *c0w, z64 *bubloc_tmp,
                               cudaStream_t st) {
-  int n = 2 * c.iwf * c.nd2 + c.nd2;
   cudaError_t e = cudaMemsetAsync(bubloc_tmp, 0, sizeof(z64) * c.nd2 * c.nd2, st);
   if (e != cudaSuccess) return e;
-  k_local_diag<<<cdiv_u(n, 128), 128, 0, st>>>(c, iwb, c0inv, c0w, bubloc_tmp);
+  k_local_diag<<<cdiv_u(2 * c.iwf * c.nd2, 128) + cdiv_u(c.nd2, 4), 128, 0, st>>>(c, iwb, c0inv, c0w, bubloc_tmp);
   return ADGA_LAUNCH_CHECK();
 }
 
 // F~ = sym(chi_loc) * diag(chi0_loc^-1) - 1 (src/main.F90:529-553), written
-// row-major: Frow[r*N + c] = F~(r, c).  chi_loc is column-major.
-__global__ void k_local_F(int N, const z64 *chi, const z64 *c0inv, z64 *Frow, int minus_one) {
+// row-major: Frow[r*N + c] = F~(r, c).  chi_loc is column-major; blockIdx.z: the channel.
+__global__ void k_local_F(int N, const z64 *chi_d, const z64 *chi_m, const z64 *c0inv, z64 *Frow_d, z64 *Frow_m,
+                          int minus_one) {
+  const z64 *chi = blockIdx.z ? chi_m : chi_d;
+  z64 *Frow = blockIdx.z ? Frow_m : Frow_d;
   __shared__ z64 A[32][33];   // A[cc][rr] = chi(r0+rr, c0+cc)
   __shared__ z64 B[32][33];   // B[rr][cc] = chi(c0+cc, r0+rr)
   int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
@@ -163,47 +179,65 @@ __global__ void k_local_F(int N, const z64 *chi, const z64 *c0inv, z64 *Frow, in
   }
 }
 
-cudaError_t launch_local_F(const DevCtx &c, const z64 *chi_loc, const z64 *c0inv, z64 *Frow,
-                           cudaStream_t st, bool minus_one) {
-  dim3 grid(cdiv_u(c.N, 32), cdiv_u(c.N, 32));
-  k_local_F<<<grid, dim3(32, 8), 0, st>>>(c.N, chi_loc, c0inv, Frow, minus_one ? 1 : 0);
+cudaError_t launch_local_F(const DevCtx &c, const z64 *chi_d, const z64 *chi_m, const z64 *c0inv, z64 *Frow_d,
+                           z64 *Frow_m, cudaStream_t st, bool minus_one) {
+  dim3 grid(cdiv_u(c.N, 32), cdiv_u(c.N, 32), 2);
+  k_local_F<<<grid, dim3(32, 8), 0, st>>>(c.N, chi_d, chi_m, c0inv, Frow_d, Frow_m, minus_one ? 1 : 0);
   return ADGA_LAUNCH_CHECK();
 }
 
 // gamma^w(i1, :) = sum_dum F~(i1 + dum*nd2, :) and 1 + gamma^w
-// (src/main.F90:564-570, 617-625); column-major (nd2, N).
-__global__ void k_local_gamma(int N, int nd2, int n2iwf, const z64 *Frow, z64 *gam, z64 *opg) {
-  size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (idx >= (size_t)nd2 * N) return;
-  int cc = (int)(idx % N), i1 = (int)(idx / N);
+// (src/main.F90:564-570, 617-625); column-major (nd2, N); blockIdx.z: the channel.
+// A warp takes 32 columns and every eighth frequency, the warps' parts are added in their order: with
+// all frequencies in one thread both channels took 20 us on N = 40, 67 us on N = 160 and 52 us on
+// N = 1080, one serial chain of loads; this form: 4 us, 8.5 us and 9.6 us.
+__global__ void __launch_bounds__(256)
+k_local_gamma(int N, int nd2, int n2iwf, const z64 *Frow_d, const z64 *Frow_m, z64 *gam_d, z64 *gam_m, z64 *opg_d,
+              z64 *opg_m) {
+  __shared__ z64 part[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, cc = blockIdx.x * 32 + lane, i1 = blockIdx.y;
+  const z64 *Frow = blockIdx.z ? Frow_m : Frow_d;
   z64 s = czero<z64>();
-  for (int dum = 0; dum < n2iwf; ++dum) s = cadd(s, Frow[(size_t)(i1 + dum * nd2) * N + cc]);
-  gam[i1 + (size_t)cc * nd2] = s;
+  if (cc < N)
+#pragma unroll 4
+    for (int dum = w; dum < n2iwf; dum += 8) s = cadd(s, Frow[(size_t)(i1 + dum * nd2) * N + cc]);
+  part[w][lane] = s;
+  __syncthreads();
+  if (w || cc >= N) return;
+  for (int v = 1; v < 8; ++v) s = cadd(s, part[v][lane]);
+  (blockIdx.z ? gam_m : gam_d)[i1 + (size_t)cc * nd2] = s;
+  if (!opg_d) return;                   // tangents: gamma only
   if (cc % nd2 == i1) s.x += 1.0;
-  opg[i1 + (size_t)cc * nd2] = s;
+  (blockIdx.z ? opg_m : opg_d)[i1 + (size_t)cc * nd2] = s;
 }
 
-cudaError_t launch_local_gamma(const DevCtx &c, const z64 *Frow, z64 *gam, z64 *opg, cudaStream_t st) {
-  size_t total = (size_t)c.nd2 * c.N;
-  k_local_gamma<<<cdiv_u(total, 256), 256, 0, st>>>(c.N, c.nd2, 2 * c.iwf, Frow, gam, opg);
+cudaError_t launch_local_gamma(const DevCtx &c, const z64 *Frow_d, const z64 *Frow_m, z64 *gam_d, z64 *gam_m,
+                               z64 *opg_d, z64 *opg_m, cudaStream_t st) {
+  k_local_gamma<<<dim3(cdiv_u(c.N, 32), c.nd2, 2), 256, 0, st>>>(c.N, c.nd2, 2 * c.iwf, Frow_d, Frow_m, gam_d, gam_m,
+                                                                opg_d, opg_m);
   return ADGA_LAUNCH_CHECK();
 }
 
 // chi_loc(w) += calc_chi_qw(gamma^w, chi0w) for both channels
-// (src/main.F90:573-577) and bubble_loc(w) += bubble_loc_tmp (:521).
+// (src/main.F90:573-577) and bubble_loc(w) += bubble_loc_tmp (:521).  A warp per
+// element, its lanes sharing the frequencies (one thread per element: 10 us on 40
+// frequencies, 47 us on 80 with four components; this form: 6.0 and 6.5 us).
 __global__ void k_chi_loc_update(DevCtx c, const z64 *gd, const z64 *gm, const z64 *c0w,
                                  const z64 *bub_tmp, z64 *cld, z64 *clm, z64 *bub_loc) {
-  int nd2 = c.nd2;
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  int nd2 = c.nd2, lane = threadIdx.x & 31;
+  int idx = blockIdx.x * 4 + (threadIdx.x >> 5);
   if (idx >= nd2 * nd2) return;
   int i1 = idx % nd2, i2 = idx / nd2;
   z64 sd = czero<z64>(), sm = czero<z64>();
-  for (int dum = 0; dum < 2 * c.iwf; ++dum) {
+  for (int dum = lane; dum < 2 * c.iwf; dum += 32) {
     z64 w = c0w[dum * nd2 + i2];
     size_t col = (size_t)(i2 + dum * nd2) * nd2;
     cfma(sd, gd[i1 + col], w);
     cfma(sm, gm[i1 + col], w);
   }
+  sd = warp_sum(sd);
+  sm = warp_sum(sm);
+  if (lane) return;
   double b2 = c.beta * c.beta;
   if (cld) {   // null with an external chi_loc: only the bubble accumulates (src/main.F90:573)
     cld[idx] = cadd(cld[idx], make_double2(sd.x / b2, sd.y / b2));
@@ -216,7 +250,7 @@ cudaError_t launch_chi_loc_update(const DevCtx &c, const z64 *gam_d, const z64 *
                                   const z64 *c0w, const z64 *bubloc_tmp, z64 *chi_loc_d,
                                   z64 *chi_loc_m, z64 *bubble_loc, cudaStream_t st) {
   int n = c.nd2 * c.nd2;
-  k_chi_loc_update<<<cdiv_u(n, 128), 128, 0, st>>>(c, gam_d, gam_m, c0w, bubloc_tmp, chi_loc_d,
+  k_chi_loc_update<<<cdiv_u(n, 4), 128, 0, st>>>(c, gam_d, gam_m, c0w, bubloc_tmp, chi_loc_d,
                                                    chi_loc_m, bubble_loc);
   return ADGA_LAUNCH_CHECK();
 }
@@ -227,8 +261,9 @@ cudaError_t launch_chi_loc_update(const DevCtx &c, const z64 *gam_d, const z64 *
 // ---------------------------------------------------------------------------
 __global__ void k_eom_static(DevCtx c, z64 *sig) {
   int nd = c.nd, nd2 = c.nd2;
-  int i = threadIdx.x;
-  if (i >= nd) return;
+  int idx = blockIdx.x * blockDim.x + threadIdx.x;      // a thread per (orbital, frequency)
+  int i = idx % nd, w = idx / nd;
+  if (w >= 2 * c.iwf) return;
   z64 t = czero<z64>();
   int i1 = i * nd + i;
   for (int j = 0; j < nd; ++j) {
@@ -237,14 +272,12 @@ __global__ void k_eom_static(DevCtx c, z64 *sig) {
     z64 f = make_double2(2.0 * a.x - b.x, 2.0 * a.y - b.y);
     cfma(t, f, c.ndmft[j]);
   }
-  for (int w = 0; w < 2 * c.iwf; ++w) {
-    size_t o = i + i * nd + (size_t)w * nd2;
-    sig[o] = cadd(sig[o], t);
-  }
+  size_t o = i + i * nd + (size_t)w * nd2;
+  sig[o] = cadd(sig[o], t);
 }
 
 cudaError_t launch_eom_static(const DevCtx &c, z64 *sigma_dmft, cudaStream_t st) {
-  k_eom_static<<<1, 32, 0, st>>>(c, sigma_dmft);
+  k_eom_static<<<cdiv_u(2 * c.iwf * c.nd, 64), 64, 0, st>>>(c, sigma_dmft);
   return ADGA_LAUNCH_CHECK();
 }
 

@@ -129,3 +129,15 @@ def test_few_points_match_transform(name, nk, nq, points):
             lad.close()
     for k in ("bubble_nl", "chi_qw_dens", "chi_qw_magn", "sigma_nl"):
         assert rel_err(got[1][k], got[0][k]) < 1e-12, (k, rel_err(got[1][k], got[0][k]))
+
+
+@pytest.mark.parametrize("nk,nq", [((1, 1, 12), (1, 1, 6)), ((20, 20, 20), (4, 2, 1)), ((7, 9, 5), (7, 3, 1)),
+                                   ((21, 20, 20), (3, 2, 1)), ((2, 2, 1500), (1, 2, 10))])
+def test_transform_meshes_match_direct(nk, nq):
+    """The one-kernel transform (up to 8192 points, axes summing to at most
+    1024) and the passes beyond it, odd axes and axes of length one: the same
+    sums as the direct kernels in another order (1e-12, as above)."""
+    p = synth.make_problem(dataclasses.replace(synth.SPECS["t1"], nk=nk, nq=nq, iwf=2, iwb=1), quick_mu=True)
+    a, b = run(p, TRANSFORM), run(p, DIRECT)
+    for k in OUT_KEYS:
+        assert rel_err(a[k], b[k]) < 1e-12, (k, rel_err(a[k], b[k]))
