@@ -8,14 +8,14 @@
 // neighbouring CTAs, the second of which finds most of the triangle in L2.
 // The streaming solves took 2.35 ms (back) and 2.73 ms (forward) for 432
 // matrices of order 1000 with 25 right-hand sides, ten times the triangle's
-// HBM time, bound by the FP32 products; these: 1.27 and 1.28 ms.  Once block p (64 rows) is
+// HBM time, bound by the FP32 products; these: 0.98 ms each.  Once block p (64 rows) is
 // solved, the rows still to solve are updated, B[rows] -= T[rows, block p] Y_p,
 // on the tensor cores, and every row block keeps its accumulated update in
 // TMEM for the whole solve:
 //   * the triangle's tiles (64 complex rows x 32 columns of one panel, 16 KB
 //     FP32) stream through a 5-stage TMA ring as they lie in memory, real
 //     and imaginary parts interleaved;
-//   * warps 4-7 split every landed tile into hi = tf32(x) (round to nearest)
+//   * warps 4-7 and 12-15 (a half tile each) split every landed tile into hi = tf32(x) (round to nearest)
 //     and lo = x - hi (exact in FP32) and write both as the K-major A
 //     operand of an M = 128 MMA whose rows are the real and imaginary parts
 //     of the 64 complex rows (kind::tf32, N = 32, K = 8 per instruction);
@@ -32,6 +32,14 @@
 //     64 x 64 block inverses of k_diag_inv, as soon as the first tile of the
 //     previous panel (the one that updates block p) has completed, so that
 //     the rest of that panel streams meanwhile.
+// Bound by HBM and, close behind, the splitting of the tiles.  What held it back
+// before: the issuing thread's descriptor arithmetic (95 clocks an MMA against
+// the 41 that one takes; now an elected thread advances precomputed ones), one
+// group of four splitting warps, and 64-long dot products per right-hand side in
+// the diagonal solve (now each element of the block inverse feeds all of them).
+// 592 matrices, us a solve: N = 1080, 9 right-hand sides 854 -> 603 (5.1 TB/s);
+// N = 320, 9: 159 -> 108; N = 320, 4: 107 -> 81; N = 160, 1: 45 -> 38.  The A
+// operands through TMEM instead of shared memory measured slower (1007 at N = 1080).
 // TMEM holds one 32-column accumulator per row block after the first solved
 // one: N <= 17 * 64 = 1088.  Every wait is bounded (WAIT_NS); on a timeout the
 // kernel records an error code in *err and returns.
@@ -48,7 +56,7 @@ namespace {
 using namespace umma;
 
 constexpr int QB = 64;                        // block width (the factorisation's NB)
-constexpr int Q_THREADS = 384;
+constexpr int Q_THREADS = 512;
 constexpr int Q_NS = 5;                       // ring stages
 constexpr int Q_KC = 32;                      // panel columns per stage
 constexpr int Q_STAGE = 128 * Q_KC * 4;       // 128 reals (64 complex rows) x 32 columns FP32 (16 KB)
@@ -63,7 +71,8 @@ constexpr int OFF_AOP = OFF_RING + Q_NS * Q_STAGE;   // two A operand pairs (hi,
 constexpr int OFF_BOP = OFF_AOP + 4 * Q_STAGE;       // two B operand pairs (hi, lo)
 constexpr int OFF_DINV = OFF_BOP + 4 * Q_BOP;
 constexpr int OFF_VST = OFF_DINV + Q_DINV;
-constexpr int OFF_BAR = OFF_VST + Q_VST;
+constexpr int OFF_PART = OFF_VST + Q_VST;            // the other half's part of Y_p, [rhs][row]
+constexpr int OFF_BAR = OFF_PART + Q_VST;
 // full[NS] empty[NS] conv[2] opfree[2] crit yready dfull done
 constexpr int Q_NBAR = 2 * Q_NS + 8;
 constexpr int Q_SMEM = OFF_BAR + 8 * Q_NBAR + 16 + 1024;
@@ -138,6 +147,8 @@ struct QGeo {
   __device__ uint32_t tcol(int j) const { return (uint32_t)((upper ? j : j - 1) * Q_NP); }
 };
 
+// RM: at least the right-hand sides of a CTA (compile-time bound of the diagonal solve's registers)
+template <int RM>
 __global__ void __launch_bounds__(Q_THREADS, 1)
 k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32 *__restrict__ Dinv, z32 *C,
           size_t strideC, int ldc, int Rtot, int nshare, int upper_i, int *err) {
@@ -168,7 +179,10 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
     for (int i = 0; i < 4; ++i) mbar_init(b_crit + 8 * i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // both B operand sets start at zero: rows n >= R (and 16 + n) are never written
+  // both B operand sets start at zero: rows n >= R (and 16 + n) are never written; so do the staged
+  // right-hand sides, whose columns from R on take part in the diagonal products
+  for (int e = t; e < Q_VST / 16; e += Q_THREADS)
+    reinterpret_cast<uint4 *>(g0 + OFF_VST)[e] = make_uint4(0u, 0u, 0u, 0u);
   for (int e = t; e < 4 * Q_BOP / 16; e += Q_THREADS)
     reinterpret_cast<uint4 *>(g0 + OFF_BOP)[e] = make_uint4(0u, 0u, 0u, 0u);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -201,29 +215,32 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
       }
     }
   } else if (warp == 1) {
-    // ---- MMA issuer
-    if (lane == 0 && nblk > 1) {
+    // ---- MMA issuer: one elected thread.  A tile's 12 MMAs (N = 32) execute in about 41 clocks each, so
+    // their descriptors are formed once and advanced by constants (16-byte units in the low word)
+    if (nblk > 1 && elect_one()) {
       bool ok = true;
       int g = 0;
+      const uint64_t da0 = desc_k(s0 + OFF_AOP), da1 = desc_k(s0 + OFF_AOP + 2 * Q_STAGE);
+      const uint64_t db0 = desc_k(s0 + OFF_BOP), db1 = desc_k(s0 + OFF_BOP + 2 * Q_BOP);
       for (int p = 0; p < nblk - 1 && ok; ++p) {
         if (!(ok = mbar_wait(b_yready, p & 1, err, 42))) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t bop = s0 + OFF_BOP + (p & 1) * 2 * Q_BOP;
+        const uint64_t dbp = (p & 1) ? db1 : db0;
         for (int tt = 0; tt < geo.ntiles(p) && ok; ++tt) {
           const uint32_t dt = tmem + geo.tcol(geo.tile_blk(p, tt));
+#pragma unroll
           for (int h = 0; h < 2; ++h, ++g) {
-            const int o = g & 1;
+            const int o = h;                          // two stages a tile: the operand pairs alternate
             if (!(ok = mbar_wait(b_conv + 8 * o, (g >> 1) & 1, err, 43))) break;
             asm volatile("tcgen05.fence::after_thread_sync;");
-            const uint32_t ahi = s0 + OFF_AOP + o * 2 * Q_STAGE, alo = ahi + Q_STAGE;
+            const uint64_t da = o ? da1 : da0;
 #pragma unroll
             for (int term = 0; term < 3; ++term)
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const uint32_t a = (term == 2 ? alo : ahi) + 32 * k;
-                const uint32_t bb = bop + (term == 1 ? Q_BOP : 0) + 4096 * h + 32 * k;
-                mma_tf32(dt, desc_k(a), desc_k(bb), (p > 0 || h > 0 || term > 0 || k > 0) ? 1u : 0u);
-              }
+              for (int k = 0; k < 4; ++k)
+                mma_tf32(dt, da + (term == 2 ? Q_STAGE / 16 : 0) + 2 * k,
+                         dbp + (term == 1 ? Q_BOP / 16 : 0) + 256 * h + 2 * k,
+                         (h > 0 || term > 0 || k > 0) ? 1u : (p > 0 ? 1u : 0u));
             mma_commit(b_opfree + 8 * o);
             if (tt == 0 && h == 1) mma_commit(b_crit);
           }
@@ -232,16 +249,16 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
       mma_commit(b_done);
       mbar_wait(b_done, 0, err, 48);
     }
-  } else if (warp >= 4 && warp < 8) {
+  } else if ((warp >= 4 && warp < 8) || warp >= 12) {
     // ---- every landed tile (128 reals x 32 columns, as loaded) into the K-major A operand pair:
     //      thread m owns row m (real index 128 j + m), hi = tf32(x), lo = x - hi
-    const int m = t - 128;
+    //      (warps 4-7 the first half of every tile, 12-15 the second)
+    const int m = t & 127, o = warp >= 12;
     bool ok = true;
-    int g = 0;
+    int g = o;
     for (int p = 0; p < nblk - 1 && ok; ++p)
-      for (int tt = 0; tt < geo.ntiles(p) && ok; ++tt)
-        for (int h = 0; h < 2; ++h, ++g) {
-          const int s = g % Q_NS, o = g & 1;
+      for (int tt = 0; tt < geo.ntiles(p) && ok; ++tt, g += 2) {
+          const int s = g % Q_NS;
           ok = mbar_wait(b_full + 8 * s, (g / Q_NS) & 1, err, 44);
           if (ok && g >= 2) ok = mbar_wait(b_opfree + 8 * o, ((g >> 1) - 1) & 1, err, 45);
           if (!ok) break;
@@ -262,7 +279,7 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           mbar_arrive(b_conv + 8 * o);
         }
-  } else if (warp >= 8) {
+  } else if (warp >= 8 && warp < 12) {
     // ---- diagonal blocks: Y_p = D_p^-1 (B_p - acc_p)
     const int dt_ = t - 256, q = warp & 3;
     float2 *vst = reinterpret_cast<float2 *>(g0 + OFF_VST);   // [rhs][row]
@@ -276,9 +293,9 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
       // this lane's right-hand-side values of block p (row r, part c), loaded before the wait for
       // the accumulator so that their latency overlaps it
       const int r = q * 16 + (lane >> 1), c = lane & 1;
-      float bv[Q_RMAX];
+      float bv[RM];
 #pragma unroll
-      for (int n = 0; n < Q_RMAX; ++n) {
+      for (int n = 0; n < RM; ++n) {
         bv[n] = 0.f;
         if (p > 0 && n < R && r < jb) bv[n] = reinterpret_cast<const float *>(Cb + (size_t)(r0 + r) + (size_t)n * ldc)[c];
       }
@@ -295,7 +312,7 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         // lane 2r: [Tr Yr | Tr Yi], lane 2r + 1: [Ti Yr | Ti Yi] of complex row r
 #pragma unroll
-        for (int n = 0; n < Q_RMAX; ++n) {
+        for (int n = 0; n < RM; ++n) {
           const float pv = __shfl_xor_sync(0xffffffffu, v[16 + n], 1);
           const float upd = c ? v[n] + pv : v[n] - pv;
           if (n < R) reinterpret_cast<float *>(vst)[(n * QB + r) * 2 + c] = r < jb ? bv[n] - upd : 0.f;
@@ -307,30 +324,45 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
         }
       }
       named_sync(1, 128);
+      // thread (row, half of k): every element of D_p^-1 read feeds all right-hand sides, every pair of V
+      // elements two rows' worth of products; the halves exchange the right-hand sides they do not store
       unsigned char *bh = g0 + OFF_BOP + (p & 1) * 2 * Q_BOP, *bl = bh + Q_BOP;
-      for (int e = dt_; e < QB * R; e += 128) {
-        const int r = e % QB, n = e / QB;
-        z32 y = make_float2(0.f, 0.f);
-        if (r < jb) {
-          // D^-1 of U is upper triangular, of the unit-lower L lower triangular
-          const int kb = geo.upper ? r : 0, ke = geo.upper ? jb : r + 1;
-          const float2 *vn = vst + n * QB;
-          z32 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
-          int k = kb;
-          for (; k + 1 < ke; k += 2) {
-            cfma(a0, D[r + k * QB], vn[k]);
-            cfma(a1, D[r + (k + 1) * QB], vn[k + 1]);
+      const int yr = dt_ & 63, hk = dt_ >> 6;
+      float2 *part = reinterpret_cast<float2 *>(g0 + OFF_PART);
+      z32 y[RM];
+#pragma unroll
+      for (int n = 0; n < RM; ++n) y[n] = make_float2(0.f, 0.f);
+      // D^-1 of U is upper triangular, of the unit-lower L lower triangular: a quarter of it is zero
+      if (geo.upper ? (hk == 1 || yr < 32) : (hk == 0 || yr >= 32)) {
+#pragma unroll 4
+        for (int k = 32 * hk; k < 32 * hk + 32; k += 2) {
+          const z32 d0 = D[yr + k * QB], d1 = D[yr + (k + 1) * QB];
+          const float2 s0v = make_float2(-d0.y, d0.y), s1v = make_float2(-d1.y, d1.y);
+#pragma unroll
+          for (int n = 0; n < RM; ++n) {
+            const float4 v = *reinterpret_cast<const float4 *>(vst + n * QB + k);
+            y[n] = __ffma2_rn(make_float2(d0.x, d0.x), make_float2(v.x, v.y), y[n]);
+            y[n] = __ffma2_rn(s0v, make_float2(v.y, v.x), y[n]);
+            y[n] = __ffma2_rn(make_float2(d1.x, d1.x), make_float2(v.z, v.w), y[n]);
+            y[n] = __ffma2_rn(s1v, make_float2(v.w, v.z), y[n]);
           }
-          if (k < ke) cfma(a0, D[r + k * QB], vn[k]);
-          y = cadd(a0, a1);
-          Cb[(size_t)(r0 + r) + (size_t)n * ldc] = y;
         }
-        const float hr = tf32_rna(y.x), hi = tf32_rna(y.y);
-        *reinterpret_cast<float *>(bh + bop_off(n, r)) = hr;
-        *reinterpret_cast<float *>(bl + bop_off(n, r)) = y.x - hr;
-        *reinterpret_cast<float *>(bh + bop_off(16 + n, r)) = hi;
-        *reinterpret_cast<float *>(bl + bop_off(16 + n, r)) = y.y - hi;
       }
+#pragma unroll
+      for (int n = 0; n < RM; ++n)
+        if ((n & 1) != hk) part[n * QB + yr] = y[n];
+      named_sync(1, 128);
+#pragma unroll
+      for (int n = 0; n < RM; ++n)
+        if ((n & 1) == hk && n < R) {
+          const z32 v = cadd(y[n], part[n * QB + yr]);
+          if (yr < jb) Cb[(size_t)(r0 + yr) + (size_t)n * ldc] = v;
+          const float hr = tf32_rna(v.x), hi = tf32_rna(v.y);
+          *reinterpret_cast<float *>(bh + bop_off(n, yr)) = hr;
+          *reinterpret_cast<float *>(bl + bop_off(n, yr)) = v.x - hr;
+          *reinterpret_cast<float *>(bh + bop_off(16 + n, yr)) = hi;
+          *reinterpret_cast<float *>(bl + bop_off(16 + n, yr)) = v.y - hi;
+        }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       named_sync(1, 128);
       if (dt_ == 0) {
@@ -371,11 +403,20 @@ cudaError_t launch_trsv_tc(const z32 *M, const LUBatch &lb, z32 *C, size_t strid
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return cudaErrorInvalidValue;
-  cudaError_t e = smem_limit(k_trsv_tc, Q_SMEM);
-  if (e != cudaSuccess) return e;
-  const int nshare = (R + Q_RMAX - 1) / Q_RMAX;
-  k_trsv_tc<<<lb.batch * nshare, Q_THREADS, Q_SMEM, st>>>(map, lb.N, lb.nsteps(),
-                                                          (const z32 *)(upper ? lb.Uinv : lb.Linv), C, strideC, ldc,
-                                                          R, nshare, upper ? 1 : 0, lb.tc_err);
+  const int nshare = (R + Q_RMAX - 1) / Q_RMAX, rper = (R + nshare - 1) / nshare;
+#define TRSV(RM)                                                                                                  \
+  do {                                                                                                            \
+    cudaError_t e = smem_limit(k_trsv_tc<RM>, Q_SMEM);                                                            \
+    if (e != cudaSuccess) return e;                                                                               \
+    k_trsv_tc<RM><<<lb.batch * nshare, Q_THREADS, Q_SMEM, st>>>(map, lb.N, lb.nsteps(),                           \
+                                                                (const z32 *)(upper ? lb.Uinv : lb.Linv), C,      \
+                                                                strideC, ldc, R, nshare, upper ? 1 : 0,           \
+                                                                lb.tc_err);                                       \
+  } while (0)
+  if (rper == 1) TRSV(1);
+  else if (rper <= 4) TRSV(4);
+  else if (rper <= 9) TRSV(9);
+  else TRSV(16);
+#undef TRSV
   return ADGA_LAUNCH_CHECK();
 }
