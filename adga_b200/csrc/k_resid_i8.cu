@@ -207,26 +207,28 @@ k_resid_i8(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    // one elected thread issues; a chunk's 56 MMAs execute in about 48 clocks each (their operands come from
+    // shared memory), so their descriptors are the stage's, advanced by constants: formed anew for each MMA
+    // they set the pace (1000 points, N = 1080: 1.69 -> 1.11 ms a channel)
+    if (elect_one()) {
       bool ok = true;
       for (int kc = 0; kc < nkc && ok; ++kc) {
         const int s = kc % NSTG;
         if (!(ok = mbar_wait(bar_full + 8 * s, (kc / NSTG) & 1, err, 32))) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t st = sbase + s * STG;
+        const uint32_t st = sbase + s * STG, more = kc > 0 ? 1u : 0u;
+        const uint64_t da = desc_sw64(st), db = desc_sw64(st + S * A_SL);
         // group g = p + q (p, q = 1..S, g <= S + 1) into accumulator g - 2
-#pragma unroll 1
+#pragma unroll
         for (int gi = 0; gi < NG; ++gi) {
           const uint32_t dacc = tmem + (uint32_t)(gi * RB_N);
-#pragma unroll 1
+#pragma unroll
           for (int p = 1; p <= gi + 1; ++p) {
             const int q = gi + 2 - p;
 #pragma unroll
-            for (int k2 = 0; k2 < 2; ++k2) {
-              const uint64_t da = desc_sw64(st + (p - 1) * A_SL + 32 * k2);
-              const uint64_t db = desc_sw64(st + S * A_SL + (q - 1) * B_SL + 32 * k2);
-              mma_i8(dacc, da, db, (kc > 0 || p > 1 || k2 > 0) ? 1u : 0u);
-            }
+            for (int k2 = 0; k2 < 2; ++k2)
+              mma_i8(dacc, da + ((p - 1) * A_SL + 32 * k2) / 16, db + ((q - 1) * B_SL + 32 * k2) / 16,
+                     p > 1 || k2 > 0 ? 1u : more);
           }
         }
         mma_commit(bar_empty + 8 * s);
