@@ -693,37 +693,46 @@ constexpr int DN_LD = 65;
 
 // Diagonal block of an unpivoted step with its inverses, one CTA per matrix
 // (FP32): the jb x jb block is padded with the identity to 64 x 64 and
-// factored right-looking in 4 x 4 register blocks, loaded straight from the
-// matrix (16 block steps, two barriers each, packed two-lane FMAs in the
-// trailing blocks; the next step's diagonal block is factored by its owner
-// right after its own trailing update, so that factorisation overlaps the
-// other blocks' updates).  L11^-1 (strictly lower; unit diagonal implied) and
-// U11^-1 (upper with the diagonal) then share one array: eight warps invert
-// the 16 x 16 diagonal blocks of both triangles (lane = column, no barriers),
-// and two levels of recursive doubling join them,
+// factored right-looking, four columns a step, its entries in registers and
+// the panel of a step in shared memory (see the body).  L11^-1 (strictly
+// lower; unit diagonal implied) and U11^-1 (upper with the diagonal) then
+// share one array: eight warps invert the 16 x 16 diagonal blocks of both
+// triangles (lane = column, no barriers), and two levels of recursive doubling
+// join them,
 //   [X00 0; X10 X11] with X10 = -X11 (L10 X00)   (and the transposed form for U),
 // 16 x 16 blocks, then 32 x 32 blocks, the products L10 X00 formed in place of
-// L10 (the factored block goes to the matrix before the inversion).  73 KB of
-// shared memory: three CTAs per SM.
-constexpr int DI_SCR = 3 * 256;
+// L10 (the factored block goes to the matrix before the inversion).  67 KB of
+// shared memory and 72 registers: three CTAs per SM.
+//
+// Bound by latency: 16 steps, each a chain of four reciprocals and two
+// barriers, and by what three CTAs read from shared memory.  An entry per
+// thread and pass (rows bi + 16 r, columns bj + 16 c) lets every warp work to
+// the end, where 4 x 4 blocks per thread left two lanes of each warp to solve
+// the panel; the factor of the next diagonal block, in a warp of its own, runs
+// beside the update (with it on the owner's path 62 instead of 56 us); scalar
+// FMAs, the packed ones cost more in moving their operands (+2 us).
+// 432 matrices (one wave) 85 -> 56 us, 2000 matrices 354 -> 237 us.
+constexpr int DI_THREADS = 288;
+constexpr int DI_SCR = 4 * 16;
 
 __device__ __forceinline__ void cfma2(z32 &acc, z32 a, z32 u) {
   acc = __ffma2_rn(make_float2(a.x, a.x), u, acc);
   acc = __ffma2_rn(make_float2(-a.y, a.y), make_float2(u.y, u.x), acc);
 }
 __device__ __forceinline__ void cfma2(z64 &acc, z64 a, z64 u) { cfma(acc, a, u); }
-// 1 / z for the FP32 block LU: z = s (a + i b) with s = max(|Re z|, |Im z|), so that
-// a^2 + b^2 lies in [1, 2]; two correctly rounded reciprocals (a zero pivot gives
-// non-finite factors, which the refinement reports)
+// 1 / z for the FP32 block LU: z = (a + i b) / s with s the power of two that brings
+// max(|a|, |b|) into [1, 2) (a result beyond the type's range apart, exact), and one correctly
+// rounded reciprocal.  A zero pivot gives non-finite factors, which the refinement reports.
 __device__ __forceinline__ z32 crcp_lu(z32 z) {
-  const float is = __frcp_rn(fmaxf(fabsf(z.x), fabsf(z.y)));
-  const float a = z.x * is, b = z.y * is;
-  const float f = __frcp_rn(fmaf(a, a, b * b)) * is;
+  const int e = __float_as_int(fmaxf(fabsf(z.x), fabsf(z.y))) & 0x7f800000;
+  const float s = __int_as_float(max(0x7f000000 - e, 0x00800000));
+  const float a = z.x * s, b = z.y * s;
+  const float f = __frcp_rn(fmaf(a, a, b * b)) * s;
   return make_float2(a * f, -b * f);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(DI_THREADS, 3)
 k_diag_inv(T *M, size_t strideM, int N, int J, int jb, int NB, int nsteps, T *Linv, T *Uinv, int *ipiv_all,
            int *rmap_all) {
   static_assert(sizeof(T) == sizeof(z32), "the blocked LU is the FP32 path's");
@@ -735,112 +744,153 @@ k_diag_inv(T *M, size_t strideM, int N, int J, int jb, int NB, int nsteps, T *Li
   const int b = blockIdx.x, t = threadIdx.x;
   T *A = M + (size_t)b * strideM;
   const T one = cx<T>::make(1, 0), zero = czero<T>();
-  const int bi = t >> 4, bj = t & 15;
-  T a[4][4];
   {
-    // thread (bi, bj) owns D[4bi.., 4bj..]: four 32-byte column pieces, all loads in flight
+    // Right-looking LU, four columns a step.  Thread (bi, bj) of warps 0..7 owns rows bi + 16 r
+    // and columns bj + 16 c.  The owners write the panel's rows and columns to D; two warps,
+    // another pair each step, solve row i of L and column i of U, one pair per thread; then
+    // every owner takes its share of A -= L U from the panel in D.  Warp 8 has factored the
+    // panel's diagonal block by then: from copies that the owners write a step ahead (nd: the
+    // next diagonal block before this step, followed by its rows and columns of the panel) it
+    // brings that block up to date while the panel is solved and factors it beside the update,
+    // so that the chain of four reciprocals, the longest of a step, is nobody else's.  Rows and
+    // columns before the current group of 16 drop out at compile time; those inside it that
+    // are already final are updated with the rest and not used again.
+    auto bar = [] { asm volatile("bar.sync 0, %0;" ::"n"(DI_THREADS) : "memory"); };
+    T *nd = S, *fd = S + 48;
+    if (t >= 256) {
+      const int lane = t & 31, r = lane & 3, c = (lane >> 2) & 3;
+      T g[4][4], rp[4];
+      bar();
+      for (int kb = 0; kb < 16; ++kb) {
+        // factor the block of step kb, every lane for itself; lane 0 writes it
+#pragma unroll
+        for (int c2 = 0; c2 < 4; ++c2)
+#pragma unroll
+          for (int r2 = 0; r2 < 4; ++r2) g[r2][c2] = fd[r2 + 4 * c2];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          rp[k] = crcp_lu(g[k][k]);
+#pragma unroll
+          for (int r2 = k + 1; r2 < 4; ++r2) g[r2][k] = cmul(g[r2][k], rp[k]);
+#pragma unroll
+          for (int r2 = k + 1; r2 < 4; ++r2)
+#pragma unroll
+            for (int c2 = k + 1; c2 < 4; ++c2) g[r2][c2] = csub(g[r2][c2], cmul(g[r2][k], g[k][c2]));
+        }
+        if (lane == 0) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            rcps[4 * kb + k] = rp[k];
+#pragma unroll
+            for (int r2 = 0; r2 < 4; ++r2) D[(4 * kb + r2) + (4 * kb + k) * DN_LD] = g[r2][k];
+          }
+        }
+        bar();
+        T l[4], u[4], v = nd[r + 4 * c];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          l[k] = nd[16 + r + 4 * k];
+          u[k] = nd[32 + k + 4 * c];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+#pragma unroll
+          for (int k2 = 0; k2 < k; ++k2) {
+            l[k] = csub(l[k], cmul(l[k2], g[k2][k]));
+            u[k] = csub(u[k], cmul(g[k][k2], u[k2]));
+          }
+          l[k] = cmul(l[k], rp[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v = csub(v, cmul(l[k], u[k]));
+        if (lane < 16) fd[r + 4 * c] = v;
+        __syncwarp();
+        bar();
+      }
+      bar();
+      return;                // the barriers below wait for the threads that are left
+    }
+    const int bi = t & 15, bj = t >> 4;
+    T a[4][4];
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        const int i = 4 * bi + r, j = 4 * bj + c;
+        const int i = bi + 16 * r, j = bj + 16 * c;
         a[r][c] = (i < jb && j < jb) ? A[(size_t)(J + i) + (size_t)(J + j) * N] : (i == j ? one : zero);
       }
-  }
-  {
-    // Right-looking LU in 4 x 4 blocks.  Per block step kb: the owner of the diagonal block
-    // has factored it (unit L, U, the reciprocals of U's diagonal) into xD; the column panel
-    // solves L[bi,kb] U_kk = A[bi,kb], the row panel L_kk U[kb,bj] = A[kb,bj]; the trailing
-    // blocks take A -= L[bi,kb] U[kb,bj] as four rank-1 updates, and the owner of block
-    // (kb + 1, kb + 1) then factors it.  Panels are exchanged through S (stride 17 per
-    // block, conflict-free for the 16 column owners of a warp).
-    T *xL = S, *xU = S + 16 * 17, *xD = S + 2 * 16 * 17;   // xD: the factored diagonal block + 1/u
-    auto factor_diag = [&](int kb) {
+    if (bi < 4 && bj < 4) fd[bi + 4 * bj] = a[0][0];
+    bar();
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const T rp = crcp_lu(a[k][k]);
-        xD[16 + k] = rp;
-        rcps[4 * kb + k] = rp;
-#pragma unroll
-        for (int i = k + 1; i < 4; ++i) a[i][k] = cmul(a[i][k], rp);
-#pragma unroll
-        for (int i = k + 1; i < 4; ++i)
-#pragma unroll
-          for (int j = k + 1; j < 4; ++j) a[i][j] = csub(a[i][j], cmul(a[i][k], a[k][j]));
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) xD[r + 4 * c] = a[r][c];
-    };
-    if (t == 0) factor_diag(0);
-    __syncthreads();
+    for (int p = 0; p < 4; ++p) {
 #pragma unroll 1
-    for (int kb = 0; kb < 16; ++kb) {
-      if (bj == kb && bi > kb) {
-        // L[bi,kb] = A[bi,kb] U_kk^-1, column by column
+      for (int q = 0; q < 4; ++q) {
+        const int k0 = 16 * p + 4 * q, qn = (q + 1) & 3;
+        const int pn = (p + 1) & 3;                      // group of the next block when q = 3
+        const bool rown = (bi >> 2) == qn, coln = (bj >> 2) == qn;
+        if ((bj >> 2) == q) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+          for (int r = p; r < 4; ++r)
+            if (r > p || bi >= 4 * q + 4) D[(bi + 16 * r) + (k0 + (bj & 3)) * DN_LD] = a[r][p];
+          if (rown) nd[16 + (bi & 3) + 4 * (bj & 3)] = q < 3 ? a[p][p] : a[pn][p];
+        }
+        if ((bi >> 2) == q) {
 #pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            T v = a[r][c];
+          for (int c = p; c < 4; ++c)
+            if (c > p || bj >= 4 * q + 4) D[(k0 + (bi & 3)) + (bj + 16 * c) * DN_LD] = a[p][c];
+          if (coln) nd[32 + (bi & 3) + 4 * (bj & 3)] = q < 3 ? a[p][p] : a[p][pn];
+        }
+        if (rown && coln) nd[(bi & 3) + 4 * (bj & 3)] = q < 3 ? a[p][p] : a[pn][pn];
+        bar();
+        const int idx = t & 63, i = k0 + 4 + idx;
+        if ((t >> 6) == q && i < 64) {
+          T l[4], u[4];
 #pragma unroll
-            for (int c2 = 0; c2 < c; ++c2) v = csub(v, cmul(a[r][c2], xD[c2 + 4 * c]));
-            a[r][c] = cmul(v, xD[16 + c]);
+          for (int c = 0; c < 4; ++c) {
+            l[c] = D[i + (k0 + c) * DN_LD];
+            u[c] = D[(k0 + c) + i * DN_LD];
           }
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+          for (int c = 0; c < 4; ++c) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) xL[bi * 17 + r + 4 * c] = a[r][c];
-      } else if (bi == kb && bj > kb) {
-        // U[kb,bj] = L_kk^-1 A[kb,bj] (unit diagonal), row by row
+            for (int c2 = 0; c2 < c; ++c2) {
+              l[c] = csub(l[c], cmul(l[c2], D[(k0 + c2) + (k0 + c) * DN_LD]));
+              u[c] = csub(u[c], cmul(D[(k0 + c) + (k0 + c2) * DN_LD], u[c2]));
+            }
+            l[c] = cmul(l[c], rcps[k0 + c]);
+          }
 #pragma unroll
-        for (int r = 1; r < 4; ++r)
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int r2 = 0; r2 < r; ++r2) a[r][c] = csub(a[r][c], cmul(xD[r + 4 * r2], a[r2][c]));
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) xU[bj * 17 + r + 4 * c] = a[r][c];
-      }
-      __syncthreads();
-      if (bi > kb && bj > kb) {
+          for (int c = 0; c < 4; ++c) {
+            D[i + (k0 + c) * DN_LD] = l[c];
+            D[(k0 + c) + i * DN_LD] = u[c];
+          }
+        }
+        bar();
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           T l[4], u[4];
 #pragma unroll
-          for (int r = 0; r < 4; ++r) l[r] = xL[bi * 17 + r + 4 * k];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) u[c] = xU[bj * 17 + k + 4 * c];
-          // a[r][c] -= l[r] u[c] as two packed FMAs per complex entry
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float2 us = make_float2(u[c].y, u[c].x);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-              a[r][c] = __ffma2_rn(make_float2(-l[r].x, -l[r].x), u[c], a[r][c]);
-              a[r][c] = __ffma2_rn(make_float2(l[r].y, -l[r].y), us, a[r][c]);
-            }
+          for (int r = p; r < 4; ++r) {
+            l[r] = D[(bi + 16 * r) + (k0 + k) * DN_LD];
+            u[r] = D[(k0 + k) + (bj + 16 * r) * DN_LD];
           }
+#pragma unroll
+          for (int c = p; c < 4; ++c)
+#pragma unroll
+            for (int r = p; r < 4; ++r) cfms(a[r][c], l[r], u[c]);
         }
-        // xD is free once the panels are solved: the next diagonal block is factored now
-        if (bi == kb + 1 && bj == kb + 1) factor_diag(kb + 1);
       }
-      __syncthreads();
     }
-    // the packed factors (multipliers below the diagonal, U on and above it) into D and the matrix
+    bar();
+    // the packed factors (multipliers below the diagonal, U on and above it) to the matrix
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        const int i = 4 * bi + r, j = 4 * bj + c;
-        D[i + j * DN_LD] = a[r][c];
-        if (i < jb && j < jb) A[(size_t)(J + i) + (size_t)(J + j) * N] = a[r][c];
+        const int i = bi + 16 * r, j = bj + 16 * c;
+        if (i < jb && j < jb) A[(size_t)(J + i) + (size_t)(J + j) * N] = D[i + j * DN_LD];
       }
   }
-  __syncthreads();
   // entries of the two inverses: L^-1 with its unit diagonal and zeros above, U^-1 with zeros below
   auto xl = [&](int r, int c) { return r > c ? X[r + c * DN_LD] : (r == c ? one : zero); };
   auto xu = [&](int r, int c) { return r <= c ? X[r + c * DN_LD] : zero; };
@@ -943,47 +993,86 @@ k_diag_inv(T *M, size_t strideM, int N, int J, int jb, int NB, int nsteps, T *Li
   __syncthreads();
   {
     // 32 -> 64: L: X10 = -X11 (L10 X00), U: Y01 = -Y00 (U01 Y11) with 32 x 32 blocks;
-    // warp w: columns 4w + q of both products, lane: row i
-    const int w = t >> 5, i = t & 31, j0 = 4 * w;
-    T vl[4], vu[4];
+    // warps 0..3 the L product, 4..7 the U product; lane: rows i, i + 16, columns j0 + q.  The
+    // products with a triangle skip its zero quarter (and, by groups of 8 columns, its zeros)
+    const int w = t >> 5, lane = t & 31, w4 = w & 3;
+    const bool up = w >= 4;
+    const int i = lane & 15, j0 = 8 * w4 + 4 * (lane >> 4);
+    T v[2][4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) vl[q] = vu[q] = zero;
-    // L10 X00: X00(k, j) = 0 for k < j
+    for (int q = 0; q < 4; ++q) v[0][q] = v[1][q] = zero;
+    if (!up) {             // L10 X00: X00(k, j) = 0 for k < j
 #pragma unroll 4
-    for (int k = j0; k < 32; ++k) {
-      const T d = D[(32 + i) + k * DN_LD];
+      for (int k = 8 * w4; k < 32; ++k) {
+        const T d0 = D[(32 + i) + k * DN_LD], d1 = D[(48 + i) + k * DN_LD];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) cfma2(vl[q], d, xl(k, j0 + q));
-    }
-    // U01 Y11: Y11(k, j) = 0 for k > j
+        for (int q = 0; q < 4; ++q) {
+          const T x = xl(k, j0 + q);
+          cfma2(v[0][q], d0, x);
+          cfma2(v[1][q], d1, x);
+        }
+      }
+    } else {               // U01 Y11: Y11(k, j) = 0 for k > j
 #pragma unroll 4
-    for (int k = 0; k < j0 + 4; ++k) {
-      const T d = D[i + (32 + k) * DN_LD];
+      for (int k = 0; k < 8 * w4 + 8; ++k) {
+        const T d0 = D[i + (32 + k) * DN_LD], d1 = D[(16 + i) + (32 + k) * DN_LD];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) cfma2(vu[q], d, xu(32 + k, 32 + j0 + q));
+        for (int q = 0; q < 4; ++q) {
+          const T x = xu(32 + k, 32 + j0 + q);
+          cfma2(v[0][q], d0, x);
+          cfma2(v[1][q], d1, x);
+        }
+      }
     }
     __syncthreads();
+    const int ro = up ? 0 : 32, co = up ? 32 : 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      D[(32 + i) + (j0 + q) * DN_LD] = vl[q];
-      D[i + (32 + j0 + q) * DN_LD] = vu[q];
-      vl[q] = vu[q] = zero;
-    }
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        D[(ro + 16 * h + i) + (co + j0 + q) * DN_LD] = v[h][q];
+        v[h][q] = zero;
+      }
     __syncthreads();
+    if (!up) {             // X11(i, k) = 0 for k > i
 #pragma unroll 4
-    for (int k = 0; k < 32; ++k) {
-      const T xa = xl(32 + i, 32 + k), xb = xu(i, k);
+      for (int k = 0; k < 16; ++k) {
+        const T x0 = xl(32 + i, 32 + k), x1 = X[(48 + i) + (32 + k) * DN_LD];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        cfma2(vl[q], xa, D[(32 + k) + (j0 + q) * DN_LD]);
-        cfma2(vu[q], xb, D[k + (32 + j0 + q) * DN_LD]);
+        for (int q = 0; q < 4; ++q) {
+          const T d = D[(32 + k) + (j0 + q) * DN_LD];
+          cfma2(v[0][q], x0, d);
+          cfma2(v[1][q], x1, d);
+        }
+      }
+#pragma unroll 4
+      for (int k = 16; k < 32; ++k) {
+        const T x1 = xl(48 + i, 32 + k);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cfma2(v[1][q], x1, D[(32 + k) + (j0 + q) * DN_LD]);
+      }
+    } else {               // Y00(i, k) = 0 for k < i
+#pragma unroll 4
+      for (int k = 0; k < 16; ++k) {
+        const T x0 = xu(i, k);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cfma2(v[0][q], x0, D[k + (32 + j0 + q) * DN_LD]);
+      }
+#pragma unroll 4
+      for (int k = 16; k < 32; ++k) {
+        const T x0 = X[i + k * DN_LD], x1 = xu(16 + i, k);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const T d = D[k + (32 + j0 + q) * DN_LD];
+          cfma2(v[0][q], x0, d);
+          cfma2(v[1][q], x1, d);
+        }
       }
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      X[(32 + i) + (j0 + q) * DN_LD] = cneg(vl[q]);
-      X[i + (32 + j0 + q) * DN_LD] = cneg(vu[q]);
-    }
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) X[(ro + 16 * h + i) + (co + j0 + q) * DN_LD] = cneg(v[h][q]);
   }
   __syncthreads();
   const size_t off = ((size_t)b * nsteps + J / NB) * NB * NB;
@@ -1414,7 +1503,7 @@ static cudaError_t nopiv_step_kernels(z32 *M, const LUBatch &lb, int J, int jb, 
   smem_limit(k_diag_inv<T>, (int)sm_di);
   smem_limit(k_tri_tile<T, true>, (int)sm_tt);
   smem_limit(k_tri_tile<T, false>, (int)sm_tt);
-  k_diag_inv<T><<<lb.batch, 256, sm_di, st>>>(M, lb.strideM, lb.N, J, jb, lb.NB, nsteps, (T *)lb.Linv,
+  k_diag_inv<T><<<lb.batch, DI_THREADS, sm_di, st>>>(M, lb.strideM, lb.N, J, jb, lb.NB, nsteps, (T *)lb.Linv,
                                               (T *)lb.Uinv, lb.ipiv, lb.rmap);
   if ((e = ADGA_LAUNCH_CHECK()) != cudaSuccess) return e;
   if (!tiles) return cudaSuccess;

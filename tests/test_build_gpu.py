@@ -46,3 +46,11 @@ def test_point_matches_oracle(ndim, iwf, with_vq, prec, tol):
     assert info == 0
     for got, key in ((ed, "etaqd"), (em, "etaqm"), (gq, "gammaqd")):
         assert rel_err(got, want[key]) < tol, (key, rel_err(got, want[key]))
+
+
+@pytest.mark.parametrize("iwf", [31, 32, 33, 48, 63, 65])
+def test_unpivoted_blocks_match_oracle(iwf):
+    """The unpivoted FP32 block LU of 64 columns at full and partial last blocks
+    (N = 62 .. 130: 62, 64, 2, 32, 62 and 2 columns), with the refinement's
+    tolerance of 1e-10 on the residual, condition numbers below 100."""
+    test_point_matches_oracle(1, iwf, False, "mixed", 1e-8)
