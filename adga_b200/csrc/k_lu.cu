@@ -588,8 +588,7 @@ k_swap_left(T *M, size_t strideM, int N, int J, const int *rmap_all) {
   swap_tile<T>(M + (size_t)b * strideM, N, cnt, cs, min(J, cs + TW) - cs, s_map);
 }
 
-template <typename T> struct TrsmOp;
-template <> struct TrsmOp<z32> {
+struct TrsmOp {
   typedef float4 L;
   typedef float4 X;
   static __device__ __forceinline__ L packL(z32 l) { return make_float4(l.x, l.x, -l.y, l.y); }
@@ -599,22 +598,15 @@ template <> struct TrsmOp<z32> {
     acc = __ffma2_rn(make_float2(l.z, l.w), make_float2(x.z, x.w), acc);
   }
 };
-template <> struct TrsmOp<z64> {
-  typedef z64 L;
-  typedef z64 X;
-  static __device__ __forceinline__ L packL(z64 l) { return l; }
-  static __device__ __forceinline__ X packX(z64 x) { return x; }
-  static __device__ __forceinline__ void fma(z64 &acc, const L &l, const X &x) { cfma(acc, l, x); }
-};
 
-template <typename T>
 __global__ void __launch_bounds__(256)
-k_swap_trsm(T *M, size_t strideM, int N, int ncols, int J, int jb, int NB, int nsteps,
-            const int *rmap_all, const T *Linv) {
-  typedef TrsmOp<T> Op;
+k_swap_trsm(z32 *M, size_t strideM, int N, int ncols, int J, int jb, int NB, int nsteps,
+            const int *rmap_all, const z32 *Linv) {
+  typedef z32 T;
+  typedef TrsmOp Op;
   extern __shared__ __align__(16) unsigned char smraw[];
-  typename Op::L *Ls = reinterpret_cast<typename Op::L *>(smraw);           // [64 k][64 i]
-  typename Op::X *Xs = reinterpret_cast<typename Op::X *>(Ls + 64 * 64);    // [TW c][TS_LD k]
+  Op::L *Ls = reinterpret_cast<Op::L *>(smraw);           // [64 k][64 i]
+  Op::X *Xs = reinterpret_cast<Op::X *>(Ls + 64 * 64);    // [TW c][TS_LD k]
   __shared__ int s_map[4 * 64];
   const int b = blockIdx.y, t = threadIdx.x;
   T *A = M + (size_t)b * strideM;
@@ -649,17 +641,17 @@ k_swap_trsm(T *M, size_t strideM, int N, int ncols, int J, int jb, int NB, int n
     int k = 0;
 #pragma unroll 2
     for (; k < ka; ++k) {
-      const typename Op::L la = Ls[ia + k * 64], lb = Ls[ib + k * 64];
+      const Op::L la = Ls[ia + k * 64], lb = Ls[ib + k * 64];
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
-        const typename Op::X x = Xs[k + (cq + 8 * n) * TS_LD];
+        const Op::X x = Xs[k + (cq + 8 * n) * TS_LD];
         Op::fma(acc[0][n], la, x);
         Op::fma(acc[1][n], lb, x);
       }
     }
 #pragma unroll 2
     for (; k < kb; ++k) {
-      const typename Op::L lb = Ls[ib + k * 64];
+      const Op::L lb = Ls[ib + k * 64];
 #pragma unroll
       for (int n = 0; n < 4; ++n) Op::fma(acc[1][n], lb, Xs[k + (cq + 8 * n) * TS_LD]);
     }
@@ -671,6 +663,115 @@ k_swap_trsm(T *M, size_t strideM, int N, int ncols, int J, int jb, int NB, int n
         for (int n = 0; n < 4; ++n) {
           const int c = cq + 8 * n;
           if (c < nc) A[(size_t)(J + i) + (size_t)(cs + c) * N] = acc[m][n];
+        }
+    }
+  }
+}
+
+// The FP64 step: the interchanges and the product in one pass over a tile.  The rows of A12
+// are fetched from where the interchanges take them (cp.async, straight to shared memory), the
+// rows that move below the panel go through registers, and U12 = L11^-1 A12 runs on the tensor
+// cores: L11^-1 as 8 x 4 fragments of its lower triangle (36 KB), staged once per CTA; warp w
+// owns the row blocks w & 3 and 7 - (w & 3), 18 fragments each pair, of two of the four column
+// blocks.  A lane reads its entries of L and of A12 as 16-byte words without bank conflicts
+// (column stride 68).  71 KB of shared memory: three CTAs per SM, one's loads behind the
+// others' products.  Bound by the FP64 tensor cores and the rows' traffic alike; the earlier
+// kernel swapped in place, read the tile back and multiplied with FMAs whose operands took
+// more shared-memory cycles than they did.  17 steps of 250 points
+// (500 matrices, N = 1080) 9.4 -> 3.6 ms, of 389 two-orbital points (N = 320) 1.47 -> 0.63 ms.
+constexpr int SD_LD = 68, SD_FRAGS = 72;
+
+__global__ void __launch_bounds__(256, 3)
+k_swap_trsm_d(z64 *M, size_t strideM, int N, int ncols, int J, int jb, int NB, int nsteps,
+              const int *rmap_all, const z64 *Linv) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  z64 *Lf = reinterpret_cast<z64 *>(smraw);      // fragment rb (rb + 1) + s: rows 8 rb.., columns 4 s..
+  z64 *Xs = Lf + SD_FRAGS * 32;                  // [TW c][SD_LD k]
+  __shared__ int s_src[64], s_od[64], s_os[64], s_n;
+  const int b = blockIdx.y, t = threadIdx.x, w = t >> 5, lane = t & 31;
+  z64 *A = M + (size_t)b * strideM;
+  const z64 *L = Linv + ((size_t)b * nsteps + J / NB) * NB * NB;
+  if (t < 64) s_src[t] = J + t;
+  if (t == 0) s_n = 0;
+  for (int s = 0; s < 2 * w + 2; ++s) {
+    const int i = 8 * w + (lane >> 2), k = 4 * s + (lane & 3);
+    Lf[(w * (w + 1) + s) * 32 + lane] = (i < jb && k <= i) ? L[i + k * NB] : czero<z64>();
+  }
+  __syncthreads();
+  {
+    // sources of the panel's rows; the rows below it (one per interchange at most)
+    const int *rm = rmap_all + (size_t)b * RMAP_STRIDE;
+    const int cnt = min(rm[0], 128);
+    if (t < cnt) {
+      const int dst = rm[1 + 2 * t], src = rm[2 + 2 * t];
+      if (dst < J + jb) {
+        s_src[dst - J] = src;
+      } else {
+        const int o = atomicAdd(&s_n, 1);
+        if (o < 64) {
+          s_od[o] = dst;
+          s_os[o] = src;
+        }
+      }
+    }
+  }
+  const int cb = 16 * (w >> 2);
+  const int kk = t & 63, cc = t >> 6;
+  for (int tile = 0; tile < TPC; ++tile) {
+    const int cs = J + jb + (blockIdx.x * TPC + tile) * TW;
+    if (cs >= ncols) break;
+    const int nc = min(ncols, cs + TW) - cs;
+    __syncthreads();               // L and the map staged; the previous tile's Xs reads are done
+    const int nout = min(s_n, 64);
+    z64 v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int c = cc + 4 * q;
+      const bool in = kk < jb && c < nc;
+      zg::cp_async16(&Xs[kk + c * SD_LD], in ? &A[(size_t)s_src[kk] + (size_t)(cs + c) * N] : A, in ? 16 : 0);
+    }
+    zg::cp_async_commit();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int c = cc + 4 * q;
+      if (kk < nout && c < nc) v[q] = A[(size_t)s_os[kk] + (size_t)(cs + c) * N];
+    }
+    zg::cp_async_wait<0>();
+    __syncthreads();               // every row of the tile has been read
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int c = cc + 4 * q;
+      if (kk < nout && c < nc) A[(size_t)s_od[kk] + (size_t)(cs + c) * N] = v[q];
+    }
+    if (cb >= nc) continue;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      const int rb = h ? 7 - (w & 3) : w & 3, r0 = 8 * rb;
+      if (r0 >= jb) continue;
+      double re[2][2] = {}, im[2][2] = {};
+      const z64 *lf = Lf + rb * (rb + 1) * 32 + lane;
+      const z64 *xs = Xs + (cb + (lane >> 2)) * SD_LD + (lane & 3);
+#pragma unroll 2
+      for (int s = 0; s < 2 * rb + 2; ++s) {
+        const z64 l = lf[s * 32];
+        const double ln = -l.y;
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          const z64 x = xs[8 * n * SD_LD + 4 * s];
+          zg::dmma(re[n], l.x, x.x);
+          zg::dmma(im[n], l.x, x.y);
+          zg::dmma(re[n], ln, x.y);
+          zg::dmma(im[n], l.y, x.x);
+        }
+      }
+      const int i = r0 + (lane >> 2);
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int c = cb + 8 * n + 2 * (lane & 3) + u;
+          if (i < jb && c < nc)
+            A[(size_t)(J + i) + (size_t)(cs + c) * N] = cx<z64>::make(re[n][u], im[n][u]);
         }
     }
   }
@@ -1568,9 +1669,7 @@ cudaError_t lu_step(T *M, const LUBatch &lb, int s, bool apply_left, trail_fn tr
   const int nsteps = lb.nsteps();
   cudaError_t e;
   const size_t sm_tri = sizeof(T) * 64 * TI_LD;
-  const size_t sm_trsm = sizeof(typename TrsmOp<T>::L) * 64 * 64 + sizeof(typename TrsmOp<T>::X) * TW * TS_LD;
   smem_limit(k_triinv<T>, 200 * 1024);
-  smem_limit(k_swap_trsm<T>, 200 * 1024);
   const int J = s * lb.NB, jb = min(lb.NB, lb.N - J);
   if constexpr (sizeof(T) == sizeof(z32)) {
     if (nopiv) {
@@ -1590,8 +1689,18 @@ cudaError_t lu_step(T *M, const LUBatch &lb, int s, bool apply_left, trail_fn tr
     if ((e = ADGA_LAUNCH_CHECK()) != cudaSuccess) return e;
   }
   if (nright > 0) {
-    k_swap_trsm<T><<<dim3((nright + TPC - 1) / TPC, lb.batch), 256, sm_trsm, st>>>(M, lb.strideM, lb.N, lb.ncols, J, jb, lb.NB,
-                                                                 nsteps, lb.rmap, (const T *)lb.Linv);
+    const dim3 grid((nright + TPC - 1) / TPC, lb.batch);
+    if constexpr (sizeof(T) == sizeof(z64)) {
+      const size_t sm = sizeof(z64) * (SD_FRAGS * 32 + TW * SD_LD);
+      smem_limit(k_swap_trsm_d, (int)sm);
+      k_swap_trsm_d<<<grid, 256, sm, st>>>(M, lb.strideM, lb.N, lb.ncols, J, jb, lb.NB, nsteps, lb.rmap,
+                                           (const z64 *)lb.Linv);
+    } else {
+      const size_t sm = sizeof(TrsmOp::L) * 64 * 64 + sizeof(TrsmOp::X) * TW * TS_LD;
+      smem_limit(k_swap_trsm, (int)sm);
+      k_swap_trsm<<<grid, 256, sm, st>>>(M, lb.strideM, lb.N, lb.ncols, J, jb, lb.NB, nsteps, lb.rmap,
+                                         (const z32 *)lb.Linv);
+    }
     if ((e = ADGA_LAUNCH_CHECK()) != cudaSuccess) return e;
   }
   return lu_trail_step<T>(M, lb, J, jb, trail, trail_ctx, st, tt);
