@@ -139,7 +139,7 @@ cudaError_t launch_identity(int n, z64 *E, cudaStream_t st);
 cudaError_t launch_init_x(const z32 *T32, size_t strideM, int N, int R, int nmat, z64 *X, cudaStream_t st);
 // rnorm (nullable): per-matrix max |re| + |im| of the FP64 residual, atomicMax on the bit patterns;
 // Bpt (nullable): per-point right-hand sides in X's layout instead of (1+gamma^w) (tangent solves)
-// ri8 (k_resid_i8.cu context, or null for the FP64 CUDA-core GEMM): the product
+// ri8 (k_resid_i8.cu context, or null for the FP64 GEMM): the product
 // X D F~ from exact int8 slices on the tensor cores; fgen names the current F~
 // (its slices are cut again when it changes)
 cudaError_t launch_residual(const DevCtx &c, int npts, const z64 *X, const z64 *chi0q,

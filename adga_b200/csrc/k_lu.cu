@@ -8,9 +8,10 @@
 //                right-looking updates of the rest of the panel;
 //   k_triinv     inverts the unit-lower and upper NB x NB diagonal blocks;
 //   k_swap_trsm  applies the panel's row interchanges to the other columns
-//                and forms U12 = L11^-1 A12 as a small GEMM;
-//   trailing     A22 -= L21 U12 (CUDA-core GEMM below, or the tensor-core
-//                BF16x3 kernel of the mixed path).
+//                and forms U12 = L11^-1 A12 as a small GEMM (FP64:
+//                k_swap_trsm_d, on the tensor cores);
+//   trailing     A22 -= L21 U12 (FP64: k_zgemm.cu; FP32: the CUDA-core GEMM
+//                below, or the tensor-core BF16x3 kernel of the mixed path).
 // Pivot choice follows izamax: the largest |re|+|im|, the lowest row on ties.
 #include "lu.cuh"
 #include "zgemm.cuh"
@@ -1567,7 +1568,7 @@ cudaError_t lu_trail_cuda(T *M, const LUBatch &lb, int J, int jb, cudaStream_t s
   return ADGA_LAUNCH_CHECK();
 }
 
-// trailing update of step (J, jb) through `trail` (or the CUDA-core GEMM), timed into tt
+// trailing update of step (J, jb) through `trail` (or the plain GEMM), timed into tt
 template <typename T>
 static cudaError_t lu_trail_step(T *M, const LUBatch &lb, int J, int jb, trail_fn trail, void *trail_ctx,
                                  cudaStream_t st, TrailTiming *tt) {

@@ -229,7 +229,7 @@ int adga_ladder_run(adga_handle *h, int qwstart, int qwstop, int precision,
  *              separate operand-split kernels
  *   batch   points per batch (0: as many as 60% of the free memory holds)
  *   resid   1: the FP64 refinement residual's product X D F~ formed exactly
- *              from int8 slices on the tensor cores; 0: FP64 CUDA-core GEMM
+ *              from int8 slices on the tensor cores; 0: FP64 GEMM
  *   trsv_tc 1: the triangular solves of the FP32 factors on the tensor cores
  *              (3-term TF32 split; N <= 1088); 0: streaming
  *              CUDA-core solves
