@@ -19,8 +19,12 @@
 //     and lo = x - hi (exact in FP32) and write both as the K-major A
 //     operand of an M = 128 MMA whose rows are the real and imaginary parts
 //     of the 64 complex rows (kind::tf32, N = 32, K = 8 per instruction);
-//     the ring slot is free again once read, the operand pair once its MMAs
-//     complete (two pairs);
+//     the ring slot is free again once a proxy fence has followed its reads,
+//     the operand pair once its MMAs complete (two pairs).  Released by an
+//     arrival right after the reads, a slot was at times overwritten before
+//     them: about one of 1000 solves of 13 right-hand sides and one of 30000
+//     of 9 had a tile of the wrong stage in it, which the refinement hid at
+//     the cost of another sweep;
 //   * the B operand holds Y_p's real parts (rows 0..15) and imaginary parts
 //     (16..31), so TMEM lane 2r accumulates [Tr Yr | Tr Yi] and lane 2r + 1
 //     [Ti Yr | Ti Yi] of complex row r; the complex update is the
@@ -253,6 +257,9 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
     // ---- every landed tile (128 reals x 32 columns, as loaded) into the K-major A operand pair:
     //      thread m owns row m (real index 128 j + m), hi = tf32(x), lo = x - hi
     //      (warps 4-7 the first half of every tile, 12-15 the second)
+    //      The groups take turns at a ring slot, so a group sees every second phase of its barrier, and a wait by
+    //      parity cannot tell phase k from k - 2: that phase k - 1 (stage g - 5) is over follows from the group's
+    //      last wait on b_opfree, for the MMAs of stage g - 4, which come after those of g - 5.
     const int m = t & 127, o = warp >= 12;
     bool ok = true;
     int g = o;
@@ -266,8 +273,6 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
           float x[Q_KC];
 #pragma unroll
           for (int k = 0; k < Q_KC; ++k) x[k] = src[k * 128 + m];
-          // the ring slot is read: the next load may land there
-          mbar_arrive(b_empty + 8 * s);
           unsigned char *ahi = g0 + OFF_AOP + o * 2 * Q_STAGE, *alo = ahi + Q_STAGE;
 #pragma unroll
           for (int k = 0; k < Q_KC; k += 4) {
@@ -276,7 +281,11 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
             *reinterpret_cast<float4 *>(alo + aop_off(m, k)) =
                 make_float4(x[k] - hv.x, x[k + 1] - hv.y, x[k + 2] - hv.z, x[k + 3] - hv.w);
           }
+          // one proxy fence for both directions: the operands are visible to the MMAs, and the slot's reads
+          // have completed before the next load may land there (that load writes through the async proxy, which
+          // an arrival alone does not order behind them)
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          mbar_arrive(b_empty + 8 * s);
           mbar_arrive(b_conv + 8 * o);
         }
   } else if (warp >= 8 && warp < 12) {
