@@ -1720,7 +1720,7 @@ cudaError_t lu_factor(T *M, const LUBatch &lb, bool apply_left, trail_fn trail, 
 template <typename T>
 static cudaError_t trisolve(const T *M, const LUBatch &lb, T *C, size_t strideC, int ldc, int R,
                             bool upper, T *work, cudaStream_t st) {
-  // FP32 factors, up to 32 right-hand sides: the tensor-core solve (k_trsv_tc.cu)
+  // FP32 factors, up to 16 right-hand sides: the tensor-core solve (k_trsv_tc.cu)
   if constexpr (sizeof(T) == sizeof(z32))
     if (trsv_tc_supported(lb, R, upper))
       return launch_trsv_tc(reinterpret_cast<const z32 *>(M), lb, reinterpret_cast<z32 *>(C), strideC, ldc, R,

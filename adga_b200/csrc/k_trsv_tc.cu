@@ -1,14 +1,13 @@
 // Triangular solves of the mixed path on the tensor cores: U X = Y and the
-// unit-lower L Y = B of the FP32 factors without row interchanges, for the
-// BSE's ndim^2 <= 25 right-hand sides (the FP64 path and the pivoted FP32
-// factors keep the streaming solves of k_trsv.cu).
+// unit-lower L Y = B of the FP32 factors without row interchanges, for
+// R <= 16 right-hand sides (the BSE's ndim^2 columns; the FP64 path and the
+// pivoted FP32 factors keep the streaming solves of k_trsv.cu, and so do 17 to
+// 32 right-hand sides: shared by two CTAs here they took 1.0 ms instead of 2.4
+// and 2.7 on 432 matrices of order 1000, but the accumulators' rounding, which
+// a fourth product does not mend, left an error 1.08 times that of the FP32
+// sums (geometric mean of 102 five-orbital blocks, up to 2.3 times)).
 //
-// Right-looking blocked solve, one CTA per matrix and up to 16 right-hand
-// sides (what the TMEM accumulators hold); 17 to 32 are shared by two
-// neighbouring CTAs, the second of which finds most of the triangle in L2.
-// The streaming solves took 2.35 ms (back) and 2.73 ms (forward) for 432
-// matrices of order 1000 with 25 right-hand sides, ten times the triangle's
-// HBM time, bound by the FP32 products; these: 0.98 ms each.  Once block p (64 rows) is
+// Right-looking blocked solve, one CTA per matrix.  Once block p (64 rows) is
 // solved, the rows still to solve are updated, B[rows] -= T[rows, block p] Y_p,
 // on the tensor cores, and every row block keeps its accumulated update in
 // TMEM for the whole solve:
@@ -151,11 +150,11 @@ struct QGeo {
   __device__ uint32_t tcol(int j) const { return (uint32_t)((upper ? j : j - 1) * Q_NP); }
 };
 
-// RM: at least the right-hand sides of a CTA (compile-time bound of the diagonal solve's registers)
+// RM: at least the right-hand sides (compile-time bound of the diagonal solve's registers)
 template <int RM>
 __global__ void __launch_bounds__(Q_THREADS, 1)
 k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32 *__restrict__ Dinv, z32 *C,
-          size_t strideC, int ldc, int Rtot, int nshare, int upper_i, int *err) {
+          size_t strideC, int ldc, int R, int upper_i, int *err) {
   extern __shared__ unsigned char smraw[];
   const uint32_t s0 = (smem_u32(smraw) + 1023u) & ~1023u;
   unsigned char *g0 = smraw + (s0 - smem_u32(smraw));
@@ -164,11 +163,10 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
   const uint32_t b_crit = b_opfree + 16, b_yready = b_crit + 8, b_dfull = b_crit + 16, b_done = b_crit + 24;
   uint32_t *tslot = reinterpret_cast<uint32_t *>(g0 + OFF_BAR + 8 * Q_NBAR);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int b = blockIdx.x / nshare, share = blockIdx.x % nshare;
-  const int rper = (Rtot + nshare - 1) / nshare, R = min(rper, Rtot - share * rper);
+  const int b = blockIdx.x;
   const QGeo geo{(N + QB - 1) / QB, upper_i != 0};
   const int nblk = geo.nblk;
-  z32 *Cb = C + (size_t)b * strideC + (size_t)share * rper * ldc;
+  z32 *Cb = C + (size_t)b * strideC;
   const z32 *Db = Dinv + (size_t)b * nsteps * QB * QB;
 
   if (t == 0) {
@@ -395,7 +393,7 @@ k_trsv_tc(const __grid_constant__ CUtensorMap tmap, int N, int nsteps, const z32
 }  // namespace
 
 bool trsv_tc_supported(const LUBatch &lb, int R, bool upper) {
-  return lb.tc_err && lb.NB == QB && R >= 1 && R <= 2 * Q_RMAX && (lb.N + QB - 1) / QB <= Q_MAXBLK && lb.N % 2 == 0 &&
+  return lb.tc_err && lb.NB == QB && R >= 1 && R <= Q_RMAX && (lb.N + QB - 1) / QB <= Q_MAXBLK && lb.N % 2 == 0 &&
          lb.strideM % 2 == 0 && (upper || lb.nopiv) && tmap_encoder() != nullptr;
 }
 
@@ -412,19 +410,17 @@ cudaError_t launch_trsv_tc(const z32 *M, const LUBatch &lb, z32 *C, size_t strid
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return cudaErrorInvalidValue;
-  const int nshare = (R + Q_RMAX - 1) / Q_RMAX, rper = (R + nshare - 1) / nshare;
 #define TRSV(RM)                                                                                                  \
   do {                                                                                                            \
     cudaError_t e = smem_limit(k_trsv_tc<RM>, Q_SMEM);                                                            \
     if (e != cudaSuccess) return e;                                                                               \
-    k_trsv_tc<RM><<<lb.batch * nshare, Q_THREADS, Q_SMEM, st>>>(map, lb.N, lb.nsteps(),                           \
-                                                                (const z32 *)(upper ? lb.Uinv : lb.Linv), C,      \
-                                                                strideC, ldc, R, nshare, upper ? 1 : 0,           \
-                                                                lb.tc_err);                                       \
+    k_trsv_tc<RM><<<lb.batch, Q_THREADS, Q_SMEM, st>>>(map, lb.N, lb.nsteps(),                                    \
+                                                       (const z32 *)(upper ? lb.Uinv : lb.Linv), C, strideC, ldc, \
+                                                       R, upper ? 1 : 0, lb.tc_err);                              \
   } while (0)
-  if (rper == 1) TRSV(1);
-  else if (rper <= 4) TRSV(4);
-  else if (rper <= 9) TRSV(9);
+  if (R == 1) TRSV(1);
+  else if (R <= 4) TRSV(4);
+  else if (R <= 9) TRSV(9);
   else TRSV(16);
 #undef TRSV
   return ADGA_LAUNCH_CHECK();

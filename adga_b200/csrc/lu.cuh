@@ -107,7 +107,7 @@ cudaError_t lu_build_perm(const LUBatch &lb, int *perm, cudaStream_t st);
 template <typename T>
 bool trsv_stream_supported(const LUBatch &lb, size_t strideC, int R, bool upper, const int *perm,
                            const T *work);
-// tensor-core solves of FP32 factors (k_trsv_tc.cu): NB = 64, R <= 32, N <= 1088 and even,
+// tensor-core solves of FP32 factors (k_trsv_tc.cu): NB = 64, R <= 16, N <= 1088 and even,
 // the forward one only without row interchanges; needs lb.tc_err
 bool trsv_tc_supported(const LUBatch &lb, int R, bool upper);
 cudaError_t launch_trsv_tc(const z32 *M, const LUBatch &lb, z32 *C, size_t strideC, int ldc, int R, bool upper,

@@ -231,7 +231,7 @@ int adga_ladder_run(adga_handle *h, int qwstart, int qwstop, int precision,
  *   resid   1: the FP64 refinement residual's product X D F~ formed exactly
  *              from int8 slices on the tensor cores; 0: FP64 GEMM
  *   trsv_tc 1: the triangular solves of the FP32 factors on the tensor cores
- *              (3-term TF32 split; N <= 1088); 0: streaming
+ *              (3-term TF32 split; N <= 1088, ndim^2 <= 16); 0: streaming
  *              CUDA-core solves
  * A new handle starts at {0, 2, 1, 0, 1, 1} (the environment switches
  * ADGA_NO_PAIRS, ADGA_TRI_TILE, ADGA_BATCH, ADGA_RESID_FP64 and
