@@ -16,7 +16,6 @@
 #include "lu.cuh"
 #include "zgemm.cuh"
 #include <algorithm>
-#include <climits>
 
 
 // ---------------------------------------------------------------------------
@@ -48,30 +47,10 @@ template <typename T, int SW> struct PanelShared {
   int piv[SW], dst[2 * SW], src[2 * SW], cnt;
 };
 
-// the largest key of the warp and the lowest row that holds it (keys 0: none)
-__device__ __forceinline__ void warp_argmax(unsigned long long &key, int &row) {
-  const unsigned hi = (unsigned)(key >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned lo = hi == mh ? (unsigned)key : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
-  const unsigned long long m = ((unsigned long long)mh << 32) | ml;
-  row = (int)__reduce_min_sync(0xffffffffu, (key == m && m) ? (unsigned)row : (unsigned)INT_MAX);
-  key = m;
-}
-
-// 1 / z with one division: z scaled by a power of two so that |z|^2 lies in [1, 32) (or below,
-// for subnormal z), exact up to the rounding of |z|^2, of the division and of the products
-__device__ __forceinline__ z64 crcp_scaled(z64 z) {
-  const int e = max(__double2hiint(z.x) & 0x7ff00000, __double2hiint(z.y) & 0x7ff00000);
-  const double s = __hiloint2double(max(0x7fe00000 - e, 0x00100000), 0);
-  const double a = z.x * s, b = z.y * s;
-  const double f = __drcp_rn(fma(a, a, b * b));
-  return make_double2(a * f * s, -b * f * s);
-}
-__device__ __forceinline__ z32 crcp_scaled(z32 z) { return crcp(z); }
-
 // the warp's candidate for column CC: the row with the largest key, put beside the key
 template <typename T, int RPT, int SW, int CC>
-__device__ __forceinline__ void panel_search(const T (&a)[RPT][SW], const int (&pos)[RPT], PanelShared<T, SW> &S,
-                                             int N, int col, unsigned long long &key, int &row) {
+__device__ __forceinline__ void panel_search(const T (&a)[RPT][SW], const int (&pos)[RPT], int N, int col,
+                                             unsigned long long &key, int &row) {
   key = 0;
   row = INT_MAX;
 #pragma unroll
@@ -126,7 +105,7 @@ __device__ __forceinline__ void panel_column(T (&a)[RPT][SW], int (&pos)[RPT], P
     const T u = prow[CC + 1 < SW ? CC + 1 : CC];
 #pragma unroll
     for (int q = 0; q < RPT; ++q) cfms(a[q][CC + 1 < SW ? CC + 1 : CC], l[q], u);
-    panel_search<T, RPT, SW, (CC + 1 < SW ? CC + 1 : CC)>(a, pos, S, N, col + 1, key, row);
+    panel_search<T, RPT, SW, (CC + 1 < SW ? CC + 1 : CC)>(a, pos, N, col + 1, key, row);
   }
 #pragma unroll
   for (int c2 = CC + 2; c2 < SW; ++c2) {
@@ -184,7 +163,7 @@ k_panel(T *M, size_t strideM, int N, int J, int jb, int *ipiv_all, int *info_all
     unsigned long long key;
 #pragma unroll
     for (int q = 0; q < RPT; ++q) pos[q] = J + t + q * nt;
-    panel_search<T, RPT, SW, 0>(a, pos, S, N, c0, key, row);
+    panel_search<T, RPT, SW, 0>(a, pos, N, c0, key, row);
     panel_columns<T, RPT, SW, 0>(a, pos, S, N, c0, sw, t, nt, ipiv, info, key, row);
     // the sub-panel back to the matrix; its L block for the solve below
 #pragma unroll

@@ -16,7 +16,6 @@
 // and 43 us.
 #include "ctx.cuh"
 #include "lu.cuh"
-#include <climits>
 
 namespace {
 
@@ -25,15 +24,6 @@ constexpr int SMEM_MAX = 208 * 1024;
 
 __host__ __device__ inline int small_ld(int N) { return N | 1; }
 size_t small_smem(int N, int R) { return sizeof(z64) * ((size_t)small_ld(N) * (N + R) + N); }
-
-// 1 / z with one division (z scaled by a power of two against overflow)
-__device__ __forceinline__ z64 rcp_scaled(z64 z) {
-  const int e = max(__double2hiint(z.x) & 0x7ff00000, __double2hiint(z.y) & 0x7ff00000);
-  const double s = __hiloint2double(max(0x7fe00000 - e, 0x00100000), 0);
-  const double a = z.x * s, b = z.y * s;
-  const double f = 1.0 / fma(a, a, b * b);
-  return make_double2(a * f * s, -b * f * s);
-}
 
 // RL rows per lane: N <= 32 RL
 template <int RL>
@@ -66,10 +56,8 @@ k_lu_small(z64 *M, size_t strideM, int N, int R, int *info_all) {
       u = (i >= k && i < N && u <= 0x7ff0000000000000ULL) ? u + 1 : 0;
       if (u > key) { key = u; row = i; }
     }
-    const unsigned hi = (unsigned)(key >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned lo = hi == mh ? (unsigned)key : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
-    const unsigned long long m = ((unsigned long long)mh << 32) | ml;
-    int p = (int)__reduce_min_sync(0xffffffffu, (key == m && m) ? (unsigned)row : (unsigned)INT_MAX);
+    warp_argmax(key, row);
+    int p = row;
     if (p == INT_MAX) p = k;                   // all NaN
     z64 piv = czero<z64>();                    // of lane p % 32
 #pragma unroll
@@ -77,10 +65,10 @@ k_lu_small(z64 *M, size_t strideM, int N, int R, int *info_all) {
       const double a = __shfl_sync(0xffffffffu, x[q].x, p & 31), b = __shfl_sync(0xffffffffu, x[q].y, p & 31);
       if (RL == 1 || q == p >> 5) piv = make_double2(a, b);
     }
-    const bool zero = m == 1;                  // the largest |re|+|im| is zero
+    const bool zero = key == 1;                // the largest |re|+|im| is zero
     if (zero && !info) info = k + 1;
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
-    const z64 r = zero ? make_double2(nan, nan) : rcp_scaled(piv);
+    const z64 r = zero ? make_double2(nan, nan) : crcp_scaled(piv);
     if (lane == 0) {
       rcps[k] = r;
       s_p[k & 1] = zero ? -1 - p : p;          // a zero pivot eliminates nothing

@@ -15,10 +15,33 @@
 // GEMMs.
 #pragma once
 #include "common.cuh"
+#include <climits>
 
 // Row-interchange map of one step, per matrix: [count, dst0, src0, dst1, src1, ...]
 // (after the step's interchanges row dst holds what row src held before).
 constexpr int RMAP_STRIDE = 520;   // >= 1 + 2 * (2 * 128) entries
+
+// the largest key of the warp and the lowest row that holds it (keys 0: none)
+__device__ __forceinline__ void warp_argmax(unsigned long long &key, int &row) {
+  const unsigned hi = (unsigned)(key >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = hi == mh ? (unsigned)key : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
+  const unsigned long long m = ((unsigned long long)mh << 32) | ml;
+  row = (int)__reduce_min_sync(0xffffffffu, (key == m && m) ? (unsigned)row : (unsigned)INT_MAX);
+  key = m;
+}
+
+// 1 / z with one division: z scaled by a power of two so that |z|^2 lies in [1, 32) (or below,
+// for subnormal z), exact up to the rounding of |z|^2, of the division and of the products.  An infinite
+// part has no such scale: Smith's form, which gives 0
+__device__ __forceinline__ z64 crcp_scaled(z64 z) {
+  const int e = max(__double2hiint(z.x) & 0x7ff00000, __double2hiint(z.y) & 0x7ff00000);
+  if (e == 0x7ff00000) return crcp(z);
+  const double s = __hiloint2double(max(0x7fe00000 - e, 0x00100000), 0);
+  const double a = z.x * s, b = z.y * s;
+  const double f = __drcp_rn(fma(a, a, b * b));
+  return make_double2(a * f * s, -b * f * s);
+}
+__device__ __forceinline__ z32 crcp_scaled(z32 z) { return crcp(z); }
 
 struct LUBatch {
   int N, ncols, batch, NB;

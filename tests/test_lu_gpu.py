@@ -46,3 +46,22 @@ def test_zero_column_is_reported(n, col):
     A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
     A[:, col] = 0.0
     assert inverse_matrix(A)[1] == col + 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,at", [(1, 0), (5, 2), (40, 0), (64, 63), (80, 41), (81, 7), (130, 129), (357, 64), (600, 300),
+                                  (1030, 1029)])
+def test_infinite_pivot_drops_its_row_and_column(n, at):
+    """The reciprocal of an infinite pivot is zero (Smith's division): the
+    inverse is that of the matrix without the row and the column, zeros in their
+    place.  Diagonally dominant, so that the row is no earlier column's pivot;
+    error bound as above, with growth 1 and condition 2."""
+    rng = np.random.default_rng(n)
+    A = (rng.uniform(-1, 1, (n, n)) + 1j * rng.uniform(-1, 1, (n, n))) / (6 * n) + np.eye(n)
+    keep = np.arange(n) != at
+    want = np.zeros_like(A)
+    want[np.ix_(keep, keep)] = np.linalg.inv(A[np.ix_(keep, keep)])
+    A[at, at] = complex(np.inf, 0.5)
+    X, ierr, _ = inverse_matrix(A)
+    assert ierr == 0
+    assert np.max(np.abs(X - want)) <= 32 * n * np.finfo(float).eps * 2
