@@ -99,7 +99,7 @@ __device__ __forceinline__ void panel_column(T (&a)[RPT][SW], int (&pos)[RPT], P
     pos[q] = pos[q] == p ? col : pos[q] == col ? p : pos[q];
     const bool below = pos[q] > col && pos[q] < N;
     if (below && !zero) a[q][CC] = cmul(a[q][CC], rcp);
-    l[q] = below && who ? a[q][CC] : czero<T>();
+    l[q] = below ? a[q][CC] : czero<T>();       // all NaN: NaN, whatever prow holds then
   }
   if (CC + 1 < SW) {
     const T u = prow[CC + 1 < SW ? CC + 1 : CC];

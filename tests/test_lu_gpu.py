@@ -65,3 +65,18 @@ def test_infinite_pivot_drops_its_row_and_column(n, at):
     X, ierr, _ = inverse_matrix(A)
     assert ierr == 0
     assert np.max(np.abs(X - want)) <= 32 * n * np.finfo(float).eps * 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [40, 100, 520, 1030])
+def test_column_of_nan_reaches_the_columns_after_it(n):
+    """No row of the column can be a pivot; its multipliers make the columns
+    after it NaN too, the zero one among them, which then is no zero pivot."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    assert inverse_matrix(A)[1] == 0         # leaves finite values where the kernel keeps its rows
+    A[:, 1] = np.nan
+    A[:, 2] = 0.0
+    X, ierr, _ = inverse_matrix(A)
+    assert ierr == 0
+    assert np.isnan(X.real).all()
