@@ -186,7 +186,22 @@ static void free_list(std::vector<void *> &list) {
   list.clear();
 }
 
-// room for `bytes` in the handle's work buffer, valid until the next call that asks for more
+// Room for `bytes` in the handle's work buffer, valid until the next call that asks for more.  An entry
+// point that asks holds a ScratchUse: on its return a buffer above the bound goes back, since the batch
+// work is sized by the memory that is free (a post_loop of three orbitals on a 40^3 mesh takes a
+// gigabyte); what the small calls need stays, so that they do not allocate.
+constexpr size_t kScratchKeep = 32 * 1024 * 1024;
+struct ScratchUse {
+  adga_handle *h;
+  explicit ScratchUse(adga_handle *handle) : h(handle) {}
+  ScratchUse(const ScratchUse &) = delete;
+  ~ScratchUse() {
+    if (h->scr_cap <= kScratchKeep) return;
+    cudaFree(h->scr);                   // waits for the device: nothing still uses it
+    h->scr = nullptr;
+    h->scr_cap = 0;
+  }
+};
 static char *scratch(adga_handle *h, size_t bytes) {
   if (h->scr_cap < bytes) {
     cudaStreamSynchronize(h->st);
@@ -649,6 +664,7 @@ extern "C" int adga_vertex_transform(adga_handle *h, int iwb, int vertex_type, i
   if (!h || !chi_loc_dens || !chi_loc_magn) return ADGA_EINVAL;
   const size_t n = (size_t)h->c.N * h->c.N;
   z64 *tmp = nullptr;
+  ScratchUse use(h);
   if (!scratch_parts(h, {{&tmp, 2 * n}})) return fail(h, ADGA_ENOMEM, "transform output");
   int r = vertex_g4(h, iwb, vertex_type, iwfmax_g4, nineq, ndims, g4_dens, g4_magn, tmp, tmp + n);
   if (!r && (download(h, chi_loc_dens, tmp, n * sizeof(z64)) != cudaSuccess ||
@@ -1794,6 +1810,7 @@ extern "C" int adga_post_loop(adga_handle *h, adga_z *sigma_sum, adga_z *sigma_l
   const size_t ns = (size_t)c.nd2 * 2 * c.iwf * c.nkp_eom, ngl = (size_t)2 * c.iwmax * c.nd2;
   const size_t nsl = (size_t)c.nd2 * 2 * c.iwf, nnk = (size_t)c.nkp_eom * c.nd2;
   z64 *sig, *sl, *gl, *nk, *n;
+  ScratchUse use(h);
   if (!scratch_parts(h, {{&sig, ns}, {&sl, nsl}, {&gl, ngl}, {&nk, nnk}, {&n, (size_t)c.nd}}))
     return fail(h, ADGA_ENOMEM, "post_loop buffers");
   cudaError_t e;
@@ -1927,6 +1944,7 @@ extern "C" int adga_bse_point(adga_handle *h, int iq, int iwb, int precision, ad
   if (r) return r;
   z64 *scr = nullptr;
   // per-point outputs: the point's slot and one scratch slot for a re-solve
+  ScratchUse use(h);
   if (!scratch_parts(h, {{&scr, (size_t)6 * h->nd4}})) return fail(h, ADGA_ENOMEM, "scratch");
   h->qidx_h[0] = iq - 1;
   int st_info[2] = {0, 0};
@@ -1958,6 +1976,7 @@ extern "C" int adga_calc_chi_qw(adga_handle *h, adga_z *chi_qw, const adga_z *in
   const DevCtx &c = h->c;
   z64 *dchi, *dim3_, *dc0;
   const size_t nI = (size_t)c.nd2 * c.N, nC = (size_t)h->nd4 * 2 * c.iwf;
+  ScratchUse use(h);
   if (!scratch_parts(h, {{&dchi, (size_t)h->nd4}, {&dim3_, nI}, {&dc0, nC}}))
     return fail(h, ADGA_ENOMEM, "calc_chi_qw buffers");
   cudaStream_t st = h->st;
@@ -1982,6 +2001,7 @@ extern "C" int adga_calc_eom_dynamic(adga_handle *h, const adga_z *etaqd, const 
   if (r) return r;
   const size_t n = (size_t)c.nd2 * c.N, ns = (size_t)c.nd2 * 2 * c.iwf * c.nkp_eom;
   z64 *X, *scr, *chi0z, *opz, *sig;
+  ScratchUse use(h);
   if (!scratch_parts(h, {{&X, 2 * n}, {&scr, 2 * (size_t)h->nd4}, {&chi0z, (size_t)h->nd4 * 2 * c.iwf}, {&opz, n},
                          {&sig, ns}}))
     return fail(h, ADGA_ENOMEM, "eom buffers");
@@ -2025,6 +2045,7 @@ extern "C" int adga_calc_eom_dmft(adga_handle *h, const adga_z *gammawd, int iwb
   if (iwb < -c.iwb || iwb > c.iwb) return ADGA_EINVAL;
   const size_t n = (size_t)c.nd2 * c.N, ns = (size_t)c.nd2 * 2 * c.iwf;
   z64 *g, *s;
+  ScratchUse use(h);
   if (!scratch_parts(h, {{&g, n}, {&s, ns}})) return fail(h, ADGA_ENOMEM, "eom_dmft buffers");
   cudaStream_t st = h->st;
   cudaError_t e = cudaMemcpyAsync(g, gammawd, sizeof(z64) * n, cudaMemcpyHostToDevice, st);
@@ -2042,6 +2063,7 @@ extern "C" int adga_calc_eom_static(adga_handle *h, int iq, adga_z *sigma_dmft) 
   DevCtx &c = h->c;
   const size_t ns = (size_t)c.nd2 * 2 * c.iwf;
   z64 *s;
+  ScratchUse use(h);
   if (!scratch_parts(h, {{&s, ns}})) return fail(h, ADGA_ENOMEM, "eom_static buffers");
   cudaStream_t st = h->st;
   cudaError_t e = cudaMemcpyAsync(s, sigma_dmft, sizeof(z64) * ns, cudaMemcpyHostToDevice, st);
