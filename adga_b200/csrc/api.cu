@@ -812,8 +812,13 @@ static size_t bytes_per_point(const adga_handle *h, int prec, int NB) {
   return b;
 }
 
+// Points of a batch at most, whatever memory holds: the kernels of a step put its two matrices a point in
+// the grid's y or z direction, which ends at 65535
+constexpr int kMaxBatch = 32767;
+
 static int ensure_work(adga_handle *h, int prec, int want) {
   const DevCtx &c = h->c;
+  want = std::min(want, kMaxBatch);
   if (h->tune.batch > 0) want = std::min(want, h->tune.batch);
   if (h->cap_prec == prec && h->cap >= want && (h->tune.batch <= 0 || h->cap <= h->tune.batch)) return 0;
   cudaStreamSynchronize(h->st);

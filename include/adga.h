@@ -227,7 +227,8 @@ int adga_ladder_run(adga_handle *h, int qwstart, int qwstop, int precision,
  *   tri_tc  1: the L21 / U12 panel products on the tensor cores, writing the
  *              update operands directly; 0: FP32 CUDA-core tile products and
  *              separate operand-split kernels
- *   batch   points per batch (0: as many as 60% of the free memory holds)
+ *   batch   points per batch (0: as many as 60% of the free memory holds,
+ *           32767 at most)
  *   resid   1: the FP64 refinement residual's product X D F~ formed exactly
  *              from int8 slices on the tensor cores; 0: FP64 GEMM
  *   trsv_tc 1: the triangular solves of the FP32 factors on the tensor cores

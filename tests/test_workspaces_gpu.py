@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from adga_b200 import Ladder, synth
+from tests.helpers import library_env, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -29,3 +30,24 @@ def test_large_work_buffers_are_given_back():
         small.close()
         lad.close()
     assert held <= KEPT + 16 * 2 ** 20        # and what the driver rounds up
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_batches_stay_within_the_grid(prec):
+    """A 32^3 q mesh (32768 points, 65536 matrices) of one orbital would fit the
+    memory as one batch; the same results as from batches of 5000 points."""
+    p = synth.make_problem(dataclasses.replace(synth.SPECS["t1"], name="w1", nk=(32,) * 3, nq=(32,) * 3, iwf=41,
+                                               iwb=0), quick_mu=True)
+    out = []
+    for settings in ({}, {"ADGA_BATCH": "5000"}):
+        with library_env(settings):
+            lad = Ladder.from_problem(p)
+            try:
+                lad.set_vertex(0, *p.vertex(0))
+                status, stats = lad.ladder_run(1, None, prec)
+                assert not status.any() and stats["points"] == 32768
+                out.append({k: np.array(v) for k, v in lad.get_outputs().items()})
+            finally:
+                lad.close()
+    for k in ("chi_qw_dens", "chi_qw_magn", "sigma_nl"):
+        assert rel_err(out[0][k], out[1][k]) < (1e-12 if prec == "fp64" else 1e-9), k
