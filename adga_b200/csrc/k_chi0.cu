@@ -91,7 +91,7 @@ k_chi0_few(DevCtx c, int iwb, const int *__restrict__ qidx, z64 *__restrict__ ou
   z64 *g1s = reinterpret_cast<z64 *>(few_smem), *g2s = g1s + 2 * KC * F::L1;
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), S = (int)cl.num_blocks();
-  const int inu = blockIdx.y, p = blockIdx.z / (ND / F::JB), j0 = blockIdx.z % (ND / F::JB) * F::JB;
+  const int inu = blockIdx.x / S, p = blockIdx.y / (ND / F::JB), j0 = blockIdx.y % (ND / F::JB) * F::JB;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int grp = warp / F::WPG, wk = warp % F::WPG, l = grp % ND, jl = grp / ND;
   const int nu = c.iwstart + inu;
@@ -185,7 +185,7 @@ static cudaError_t launch_chi0_few(const DevCtx &c, int iwb, const int *qidx, in
   cudaError_t e = smem_limit(k_chi0_few<ND>, (int)F::SMEM);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(S, nnu_all, npts * (ND / F::JB));
+  cfg.gridDim = dim3(S * nnu_all, npts * (ND / F::JB));      // a big box has more frequencies than y holds
   cfg.blockDim = dim3(F::NT);
   cfg.dynamicSmemBytes = F::SMEM;
   cfg.stream = st;

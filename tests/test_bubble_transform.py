@@ -141,3 +141,18 @@ def test_transform_meshes_match_direct(nk, nq):
     a, b = run(p, TRANSFORM), run(p, DIRECT)
     for k in OUT_KEYS:
         assert rel_err(a[k], b[k]) < 1e-12, (k, rel_err(a[k], b[k]))
+
+
+def test_more_frequencies_than_a_grid_dimension():
+    """A big box of 65998 frequencies, one point by the direct sums and by the
+    transform (1e-12, as above)."""
+    p = synth.make_problem(dataclasses.replace(synth.SPECS["t1"], nk=(2, 2, 2), iwmax=33000, iwb=1), quick_mu=True)
+    got = []
+    for settings in (TRANSFORM, DIRECT):
+        lad = make_ladder(p, settings, bubble_big_box=True)
+        try:
+            lad.ladder_run(10, 10, "fp64")
+            got.append(lad.get_outputs()["bubble_nl"].copy())
+        finally:
+            lad.close()
+    assert rel_err(got[1], got[0]) < 1e-12
