@@ -14,7 +14,6 @@
 #include <map>
 #include <mutex>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <utility>
 #include <vector>
@@ -292,7 +291,7 @@ static cudaError_t download(adga_handle *h, void *dst, const void *src, size_t b
   int started = 1;                                   // the caller's own share is 0
   try {
     for (; started < kStageThreads; ++started) th[started] = std::thread(work, started);
-  } catch (const std::system_error &) {
+  } catch (...) {                                    // no thread, or no memory for one: nothing may leave a C entry
   }
   work(0);
   for (int w = started; w < kStageThreads; ++w) work(w);     // threads that could not be started

@@ -51,3 +51,29 @@ def test_batches_stay_within_the_grid(prec):
                 lad.close()
     for k in ("chi_qw_dens", "chi_qw_magn", "sigma_nl"):
         assert rel_err(out[0][k], out[1][k]) < (1e-12 if prec == "fp64" else 1e-9), k
+
+
+def test_large_results_into_pageable_memory():
+    """42 x 8000 numbers (5.4 MB, ten chunks of 512 KB and a part of one) go
+    through four threads' staging into pageable memory, directly into
+    page-locked: the same bytes, each time others, with fresh and reused arrays."""
+    p = synth.make_problem(dataclasses.replace(synth.SPECS["t1"], name="w3", nk=(20,) * 3, nq=(2,) * 3, iwf=21,
+                                               iwb=0), quick_mu=True)
+    lad = Ladder.from_problem(p)
+    try:
+        lad.set_vertex(0, *p.vertex(0))
+        lad.ladder_run(1, None, "fp64")
+        pinned = {k: torch.zeros(tuple(reversed(v)), dtype=torch.complex128, pin_memory=True).numpy().T
+                  for k, v in lad.output_shapes(8).items()}
+        reused = {k: np.zeros(v, complex, order="F") for k, v in lad.output_shapes(8).items()}
+        last = None
+        for _ in range(6):
+            lad.ladder_run(1, None, "fp64")           # the sums go on: another self-energy each time
+            want = lad.get_outputs(pinned)["sigma_nl"]
+            assert want.nbytes == 5376000 and np.abs(want).min() > 0
+            assert last is None or not np.array_equal(want, last)
+            last = want.copy()
+            assert np.array_equal(lad.get_outputs()["sigma_nl"], last)
+            assert np.array_equal(lad.get_outputs(reused)["sigma_nl"], last)
+    finally:
+        lad.close()
