@@ -113,11 +113,9 @@ k_bse_build(DevCtx c, int npts, int ch, const z64 *__restrict__ chi0q, const z64
       const int k = e >> 6, col = e & 63;
       const bool in = c0 + col < N;
       const z64 *g = F + (size_t)(k + nu * ND2) * N + c0 + col;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                       (unsigned)__cvta_generic_to_shared(Bs + buf * L::B_ELEMS + k * L::LDB + col)),
-                   "l"(in ? g : F), "r"(in ? 16 : 0));
+      zg::cp_async16(Bs + buf * L::B_ELEMS + k * L::LDB + col, in ? g : F, in ? 16 : 0);
     }
-    asm volatile("cp.async.commit_group;");
+    zg::cp_async_commit();
   };
   // this thread's elements of sw: (row, i3) with i1 fastest, as chi0^q lies in memory
   z64 pq[NE], pv[NE];

@@ -6,6 +6,7 @@
 // MACs per gathered 16-byte G(k-q) value; the G-table slices it reads stay in
 // L2 across the batch) and k_chi0_few for a few points.
 #include "ctx.cuh"
+#include "zgemm.cuh"
 #include <cooperative_groups.h>
 #include <algorithm>
 
@@ -99,25 +100,22 @@ k_chi0_few(DevCtx c, int iwb, const int *__restrict__ qidx, z64 *__restrict__ ou
   const z64 *g2t = (g2tab ? g2tab : c.gtab) + (size_t)(nu - iwb - c.nu_lo) * c.nkp * ND2 + j0 * ND;
   const int *kq = c.kq + (size_t)qidx[p] * c.nkp;
   const int nch = (c.nkp + KC - 1) / KC;
-  auto cp16 = [](z64 *dst, const z64 *src, bool in) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(in ? 16 : 0));
-  };
   auto load = [&](int ch, int buf) {
     if (ch < nch) {
       const int k0 = ch * KC;
       for (int e = t; e < KC * NB; e += NT) {
         const int kk = e / NB, b = e % NB;
         const bool in = k0 + kk < c.nkp;
-        cp16(g2s + (buf * KC + kk) * F::L2 + b, in ? g2t + (size_t)__ldg(kq + k0 + kk) * ND2 + b : g2t, in);
+        zg::cp_async16(g2s + (buf * KC + kk) * F::L2 + b, in ? g2t + (size_t)__ldg(kq + k0 + kk) * ND2 + b : g2t,
+                       in ? 16 : 0);
       }
       for (int e = t; e < KC * ND2; e += NT) {
         const int kk = e / ND2, a = e % ND2;
         const bool in = k0 + kk < c.nkp;
-        cp16(g1s + (buf * KC + kk) * F::L1 + a, in ? g1t + (size_t)k0 * ND2 + e : g1t, in);
+        zg::cp_async16(g1s + (buf * KC + kk) * F::L1 + a, in ? g1t + (size_t)k0 * ND2 + e : g1t, in ? 16 : 0);
       }
     }
-    asm volatile("cp.async.commit_group;");
+    zg::cp_async_commit();
   };
   z64 acc[ND][ND];                       // [i][k']
 #pragma unroll
@@ -128,7 +126,7 @@ k_chi0_few(DevCtx c, int iwb, const int *__restrict__ qidx, z64 *__restrict__ ou
   int buf = 0;
   for (int ch = rank; ch < nch; ch += S, buf ^= 1) {
     load(ch + S, buf ^ 1);
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    zg::cp_async_wait<1>();
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < KC / (32 * F::WPG); ++k) {

@@ -800,7 +800,6 @@ __device__ __forceinline__ void cfma2(z32 &acc, z32 a, z32 u) {
   acc = __ffma2_rn(make_float2(a.x, a.x), u, acc);
   acc = __ffma2_rn(make_float2(-a.y, a.y), make_float2(u.y, u.x), acc);
 }
-__device__ __forceinline__ void cfma2(z64 &acc, z64 a, z64 u) { cfma(acc, a, u); }
 // 1 / z for the FP32 block LU: z = (a + i b) / s with s the power of two that brings
 // max(|a|, |b|) into [1, 2) (a result beyond the type's range apart, exact), and one correctly
 // rounded reciprocal.  A zero pivot gives non-finite factors, which the refinement reports.

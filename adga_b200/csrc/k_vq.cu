@@ -97,17 +97,16 @@ cudaError_t launch_eom_static_vq(const DevCtx &c, const int *qidx, int npts, z64
 // 512 threads and the frequencies split: 46 us)
 constexpr int VQ_THREADS = 512;
 __global__ void __launch_bounds__(VQ_THREADS)
-k_vq_resid_extra(DevCtx c, const int *__restrict__ qidx, const z64 *__restrict__ X, const z64 *__restrict__ chi0q,
-                 const z64 *__restrict__ opg_d, z64 *__restrict__ extra) {
+k_vq_resid_extra(DevCtx c, int ns, const int *__restrict__ qidx, const z64 *__restrict__ X,
+                 const z64 *__restrict__ chi0q, const z64 *__restrict__ opg_d, z64 *__restrict__ extra) {
   extern __shared__ z64 sy[];                  // Z then Y, nd2 x nd2 each, then the parts of Z
   const int p = blockIdx.x, nd2 = c.nd2, nd4 = nd2 * nd2, N = c.N, t = threadIdx.x;
   const size_t per = (size_t)nd2 * N;
   const z64 *x = X + (size_t)(2 * p) * per;
   const z64 *cq = chi0q + (size_t)p * nd4 * 2 * c.iwf;
   z64 *Z = sy, *Y = sy + nd4, *P = Y + nd4;
-  // Z(i1, n) = sum_nu sum_m X(i1, nu nd2 + m) chi0q(m, n, nu): the frequencies shared by as many slices
-  // as the block's threads allow, added in slice order
-  const int ns = max(1, VQ_THREADS / nd4);
+  // Z(i1, n) = sum_nu sum_m X(i1, nu nd2 + m) chi0q(m, n, nu): the frequencies shared by ns slices, added in
+  // slice order
   for (int e = t; e < nd4 * ns; e += blockDim.x) {
     const int i1 = e % nd2, n = e / nd2 % nd2, sl = e / nd4;
     z64 s = make_double2(0.0, 0.0);
@@ -144,8 +143,8 @@ k_vq_resid_extra(DevCtx c, const int *__restrict__ qidx, const z64 *__restrict__
 cudaError_t launch_vq_resid_extra(const DevCtx &c, int npts, const int *qidx, const z64 *X, const z64 *chi0q,
                                   const z64 *opg_d, z64 *extra, cudaStream_t st) {
   if (npts <= 0) return cudaSuccess;
-  const int nd4 = c.nd2 * c.nd2;
-  k_vq_resid_extra<<<npts, VQ_THREADS, sizeof(z64) * nd4 * (2 + std::max(1, VQ_THREADS / nd4)), st>>>(
-      c, qidx, X, chi0q, opg_d, extra);
+  // slices: as many as the block's threads allow, no more than there are frequencies
+  const int nd4 = c.nd2 * c.nd2, ns = std::min(std::max(1, VQ_THREADS / nd4), 2 * c.iwf);
+  k_vq_resid_extra<<<npts, VQ_THREADS, sizeof(z64) * nd4 * (2 + ns), st>>>(c, ns, qidx, X, chi0q, opg_d, extra);
   return ADGA_LAUNCH_CHECK();
 }
