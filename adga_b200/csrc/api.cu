@@ -119,6 +119,7 @@ struct adga_handle {
   size_t scr_cap = 0;
   std::vector<cudaEvent_t> events;
   char *stage = nullptr;
+  size_t pageable = 0;            // bytes of large downloads before that buffer was worth its allocation
   cudaEvent_t stage_ev[2 * 4] = {};
   // last-run statistics
   adga_run_stats stats{};
@@ -240,11 +241,14 @@ static cudaEvent_t *batch_events(adga_handle *h, size_t n) {
 }
 
 // Device to host on the handle's stream.  A large copy into pageable memory would run through the
-// driver's own staging on one thread, which also takes the page faults of a fresh array (21 MB: 5.2 ms);
-// four threads with two page-locked chunks each copy and fault in parallel (2.6 ms).  Complete on return
-// in that case; smaller or page-locked copies stay asynchronous.
+// driver's own staging on one thread, which also takes the page faults of a fresh array; four threads with
+// two page-locked chunks each copy and fault in parallel (21 MB into fresh arrays: 2.7 -> 2.2 ms).  Complete
+// on return in that case; smaller or page-locked copies stay asynchronous.  Page-locked memory takes 2 to
+// 13 ms to allocate, whatever its size: a handle gets it once the copies it made without would have saved
+// as much, so that one that is used once is not slower for it.
 constexpr int kStageThreads = 4;
 constexpr size_t kStageChunk = 512 * 1024, kStageMin = 4 * 1024 * 1024;
+constexpr size_t kStageAfter = 256 * 1024 * 1024;
 static cudaError_t download(adga_handle *h, void *dst, const void *src, size_t bytes) {
   cudaPointerAttributes at{};
   if (bytes < kStageMin || cudaPointerGetAttributes(&at, dst) != cudaSuccess ||
@@ -253,6 +257,7 @@ static cudaError_t download(adga_handle *h, void *dst, const void *src, size_t b
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->st);
   }
   if (!h->stage) {
+    if ((h->pageable += bytes) <= kStageAfter) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->st);
     if (cudaMallocHost(&h->stage, 2 * kStageThreads * kStageChunk) != cudaSuccess) {
       cudaGetLastError();
       h->stage = nullptr;

@@ -54,9 +54,10 @@ def test_batches_stay_within_the_grid(prec):
 
 
 def test_large_results_into_pageable_memory():
-    """42 x 8000 numbers (5.4 MB, ten chunks of 512 KB and a part of one) go
-    through four threads' staging into pageable memory, directly into
-    page-locked: the same bytes, each time others, with fresh and reused arrays."""
+    """42 x 8000 numbers (5.4 MB, ten chunks of 512 KB and a part of one) go into
+    pageable memory through the driver for the handle's first 256 MB and through
+    four threads' staging after, directly into page-locked: the same bytes, each
+    time others, with fresh and reused arrays."""
     p = synth.make_problem(dataclasses.replace(synth.SPECS["t1"], name="w3", nk=(20,) * 3, nq=(2,) * 3, iwf=21,
                                                iwb=0), quick_mu=True)
     lad = Ladder.from_problem(p)
@@ -67,7 +68,7 @@ def test_large_results_into_pageable_memory():
                   for k, v in lad.output_shapes(8).items()}
         reused = {k: np.zeros(v, complex, order="F") for k, v in lad.output_shapes(8).items()}
         last = None
-        for _ in range(6):
+        for _ in range(40):                           # 2 x 40 copies, 430 MB
             lad.ladder_run(1, None, "fp64")           # the sums go on: another self-energy each time
             want = lad.get_outputs(pinned)["sigma_nl"]
             assert want.nbytes == 5376000 and np.abs(want).min() > 0
