@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <mutex>
 #include <string>
@@ -52,6 +53,12 @@ static cudaError_t tc_tri_fn(void *r, int J, int jb, int set, cudaStream_t st) {
 // Refinement stop on an estimate: the next correction d = r A^-1 is taken as at
 // most kEstSafety * rho * max|r| (rho from the first sweep)
 constexpr double kEstSafety = 10.0;
+// a correction's (or its bound's) size beside max|X|: NaN, which no tolerance admits, where X is not finite
+// (factors of a zero pivot, or a matrix beyond FP32's range)
+static double rel_to(double d, double xmax) {
+  if (!std::isfinite(xmax)) return std::numeric_limits<double>::quiet_NaN();
+  return xmax > 0 ? d / xmax : d;
+}
 
 struct TanState;
 struct TanWork;
@@ -1150,7 +1157,7 @@ static int tan_solve_mixed(adga_handle *h, z32 *T, const LUBatch &lb, const z64 
       for (int m = 0; m < nmat && all; ++m) {
         if (skip[m]) continue;
         const double est = kEstSafety * std::max(rho[m], 1.0) * bits(nh[2 * nmat + m]);
-        if (!((xmax[m] > 0 ? est / xmax[m] : est) <= h->tol)) all = false;
+        if (!(rel_to(est, xmax[m]) <= h->tol)) all = false;
       }
       if (all) {
         h->stats.max_refine_iters = std::max(h->stats.max_refine_iters, it + 1);
@@ -1175,7 +1182,7 @@ static int tan_solve_mixed(adga_handle *h, z32 *T, const LUBatch &lb, const z64 
         const double r1 = bits(nh[2 * nmat + m]);
         rho[m] = r1 > 0 ? md / r1 : 1.0;
       }
-      const double rel = mx > 0 ? md / mx : md;
+      const double rel = rel_to(md, mx);
       if (!skip[m] && !(rel <= h->tol)) {
         ++nbad;
         if (!(rel <= wrel)) { wrel = rel; wbad = m; }
@@ -1418,7 +1425,7 @@ static int run_batch(adga_handle *h, int iwb, int np, int off, int prec, int *st
         double west = 0.0;
         for (int m = 0; m < nmat && all; ++m) {
           const double est = kEstSafety * std::max(rho[m], 1.0) * bits(nh[2 * nmat + m]);
-          const double rel = xmax[m] > 0 ? est / xmax[m] : est;
+          const double rel = rel_to(est, xmax[m]);
           if (!(rel <= h->tol)) all = false;
           if (!(rel <= west)) west = rel;
         }
@@ -1443,7 +1450,7 @@ static int run_batch(adga_handle *h, int iwb, int np, int off, int prec, int *st
       worst = 0.0;
       for (int m = 0; m < nmat; ++m) {
         const double md = bits(nh[2 * m]), mx = bits(nh[2 * m + 1]);
-        double rel = mx > 0 ? md / mx : md;
+        const double rel = rel_to(md, mx);
         if (!(rel <= h->tol)) all = false;
         conv[m] = rel <= h->tol;
         if (!(rel <= worst)) worst = rel;

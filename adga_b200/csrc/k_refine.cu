@@ -99,7 +99,10 @@ k_xd(DevCtx c, const z64 *__restrict__ X, const z64 *__restrict__ chi0q, const z
       XD[base + (size_t)(ch * ND2 + ib + ND * r) * N + g * ND2 + jb + ND * s] = acc[r][s];
 }
 
-// X += up(V); per-matrix max |d| and max |X| (|re|+|im|) into norms[2*m], norms[2*m+1]
+// max that keeps a NaN (fmax drops it, and a point whose factors are not finite would pass for converged)
+__device__ __forceinline__ double nanmax(double a, double b) { return b > a || b != b ? b : a; }
+
+// X += up(V); per-matrix max |d| and max |X| (|re|+|im|, NaN if any is) into norms[2*m], norms[2*m+1]
 __global__ void k_update(int per, const z32 *V, z64 *X, unsigned long long *norms, const int *active) {
   const int m = blockIdx.y;
   if (active && !active[m]) return;
@@ -110,18 +113,18 @@ __global__ void k_update(int per, const z32 *V, z64 *X, unsigned long long *norm
     z64 x = X[(size_t)m * per + e];
     x.x += d.x; x.y += d.y;
     X[(size_t)m * per + e] = x;
-    md = fmax(md, fabs(d.x) + fabs(d.y));
-    mx = fmax(mx, fabs(x.x) + fabs(x.y));
+    md = nanmax(md, fabs(d.x) + fabs(d.y));
+    mx = nanmax(mx, fabs(x.x) + fabs(x.y));
   }
   for (int o = 16; o > 0; o >>= 1) {
-    md = fmax(md, __shfl_xor_sync(0xffffffffu, md, o));
-    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    md = nanmax(md, __shfl_xor_sync(0xffffffffu, md, o));
+    mx = nanmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   }
   if ((threadIdx.x & 31) == 0) { sd[threadIdx.x >> 5] = md; sx[threadIdx.x >> 5] = mx; }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) { md = fmax(md, sd[w]); mx = fmax(mx, sx[w]); }
-    // non-negative doubles order like their bit patterns
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) { md = nanmax(md, sd[w]); mx = nanmax(mx, sx[w]); }
+    // non-negative doubles order like their bit patterns, a NaN of either sign above them
     atomicMax(norms + 2 * m, (unsigned long long)__double_as_longlong(md));
     atomicMax(norms + 2 * m + 1, (unsigned long long)__double_as_longlong(mx));
   }

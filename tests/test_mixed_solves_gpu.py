@@ -69,3 +69,29 @@ def test_first_solve_is_as_good_as_streaming(ndim, iwf):
         finally:
             lad.close()
     assert 0 < first[0] <= 2 * first[1] and first[1] <= 2 * first[0]
+
+
+@pytest.mark.parametrize("name", ["t1", "t2", "t3m", "t5"])
+@pytest.mark.parametrize("exact", ["0", "1"])
+def test_points_without_finite_factors_are_solved_in_fp64(name, exact):
+    """A vertex beyond FP32's range leaves the FP32 factors without a finite entry:
+    no correction is small beside them, and every point is solved again in FP64,
+    to a FP64 run's results (same inputs, tolerance for another batch's sums)."""
+    p = synth.make_problem(name)
+    npts = p.spec.nqp * (2 * p.spec.iwb + 1)
+    outs = []
+    for precision in ("mixed", "fp64"):
+        with library_env({"ADGA_REFINE_EXACT": exact}):
+            lad = Ladder.from_problem(p)
+        try:
+            for iwb in range(-p.spec.iwb, p.spec.iwb + 1):
+                lad.set_vertex(iwb, *(1e40 * np.asarray(v) for v in p.vertex(iwb)))
+            status, stats = lad.ladder_run(1, None, precision)
+            outs.append({k: np.array(v) for k, v in lad.get_outputs().items()})
+        finally:
+            lad.close()
+        assert stats["mixed_fallbacks"] == (npts if precision == "mixed" else 0)
+        assert (status == (-1 if precision == "mixed" else 0)).all()
+    for k in ("chi_qw_dens", "chi_qw_magn", "sigma_nl"):
+        assert np.isfinite(outs[0][k]).all(), k
+        assert rel_err(outs[0][k], outs[1][k]) < 1e-10, k
