@@ -31,14 +31,17 @@ __device__ __forceinline__ void warp_argmax(unsigned long long &key, int &row) {
 }
 
 // 1 / z with one division: z scaled by a power of two so that |z|^2 lies in [1, 32) (or below,
-// for subnormal z), exact up to the rounding of |z|^2, of the division and of the products.  An infinite
-// part has no such scale: Smith's form, which gives 0
+// for subnormal z), exact up to the rounding of |z|^2, of the division and of the products.  One
+// infinite part counts as 1 beside the reciprocal 0, so that 1 / z is 0 as by Smith's form (selects: the
+// unrolled columns of a panel with that form's divisions in a branch took 1 to 2 % longer)
 __device__ __forceinline__ z64 crcp_scaled(z64 z) {
-  const int e = max(__double2hiint(z.x) & 0x7ff00000, __double2hiint(z.y) & 0x7ff00000);
-  if (e == 0x7ff00000) return crcp(z);
+  const int ex = __double2hiint(z.x) & 0x7ff00000, ey = __double2hiint(z.y) & 0x7ff00000, e = max(ex, ey);
   const double s = __hiloint2double(max(0x7fe00000 - e, 0x00100000), 0);
-  const double a = z.x * s, b = z.y * s;
+  double a = z.x * s, b = z.y * s;
   const double f = __drcp_rn(fma(a, a, b * b));
+  const bool inf = e == 0x7ff00000;        // or NaN, which f carries to both parts
+  a = inf && ey < ex ? copysign(1.0, a) : a;
+  b = inf && ex < ey ? copysign(1.0, b) : b;
   return make_double2(a * f * s, -b * f * s);
 }
 __device__ __forceinline__ z32 crcp_scaled(z32 z) { return crcp(z); }
