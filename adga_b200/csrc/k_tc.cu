@@ -446,7 +446,9 @@ k_tc_persist(const __grid_constant__ PMaps maps, z32 *M, size_t strideM, int N, 
             }
           }
         }
-        // this warp is done with the C half
+        // this warp is done with the C half: its reads before the next load's writes, which come through the
+        // async proxy
+        fence_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_cempty);
       }
