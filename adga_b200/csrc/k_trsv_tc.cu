@@ -40,8 +40,8 @@
 // the 41 that one takes; now an elected thread advances precomputed ones), one
 // group of four splitting warps, and 64-long dot products per right-hand side in
 // the diagonal solve (now each element of the block inverse feeds all of them).
-// 592 matrices, us a solve: N = 1080, 9 right-hand sides 854 -> 603 (5.1 TB/s);
-// N = 320, 9: 159 -> 108; N = 320, 4: 107 -> 81; N = 160, 1: 45 -> 38.  The A
+// 592 matrices, us a solve: N = 1080, 9 right-hand sides 854 -> 632 (4.8 TB/s);
+// N = 320, 9: 159 -> 104; N = 320, 4: 107 -> 82; N = 160, 1: 45 -> 41.  The A
 // operands through TMEM instead of shared memory measured slower (1007 at N = 1080).
 // TMEM holds one 32-column accumulator per row block after the first solved
 // one: N <= 17 * 64 = 1088.  Every wait is bounded (WAIT_NS); on a timeout the
